@@ -33,7 +33,7 @@ def available() -> bool:
 def build() -> str | None:
     """Compile libelemref.so from the reference sources (only where they are
     present); returns the library path, or None without the sources."""
-    if not os.path.isdir(REF_SRC):
+    if not os.path.isfile(os.path.join(REF_SRC, "src", "core", "global.cpp")):
         return LIB if available() else None
     subprocess.run(["make", "-s", "-j", str(os.cpu_count() or 4), "-C", os.path.join(_HERE, "refbuild"),
                     f"REF={REF_SRC}"], check=True)

@@ -1,49 +1,65 @@
 // Register-resident LU panel (lu::Panel, lapack-like/LU/Panel.hpp:19-89).
 //
 // One thread-block cluster of P <= 16 CTAs of 256 threads; CTA c owns rows
-// [c R, c R + R), R = RT * 256, and thread t of the CTA owns local rows
-// t, t + 256, ... (RT of them).  The panel is processed in 16-column
-// sub-panels; a thread keeps the 16 sub-panel entries of each of its rows in
-// registers.  Registers cannot be indexed at run time, so the 16-column loop
-// is unrolled: column t of the sub-panel is register t, and the rank-1 update
-// of column t touches registers t + 1 .. 15 only.
+// [c R, c R + R) (R a multiple of 16), the first CT = 32 CW threads of the CTA
+// (its column threads) own local rows t, t + CT, ... (RT of them); the other
+// warps help between the sub-panels.  The panel is processed in 16-column
+// sub-panels; a column thread keeps its rows' sub-panel entries in registers, and each column step rotates them by one as part of its rank-1
+// update, v[k] := v[k + 1] - l u[k], so that register 0 is always the current
+// column, the column loop stays rolled, and the columns already done have
+// rotated out as zeros (the winner's u needs no masking).
 //
-// Per column (one __syncthreads and one local mbarrier wait):
-//  1. each warp finds its first maximal |a| over rows >= j with three
-//     redux.sync reductions (|a| as an order-preserving 64-bit key, then the
-//     lowest row among equal keys); the lane that owns the candidate stages
-//     its 16-entry row and the reciprocal of its pivot in shared memory;
-//  2. warps 0 and 1 pick the CTA's candidate from the 8 warp candidates and
-//     store the message (candidate, its row, its reciprocal, and row j from
-//     the CTA that owns row j) into every CTA's shared memory with
-//     asynchronous stores (st.async), four lanes per destination, counted in
-//     bytes on the destination's mbarrier for this column (each CTA arms its
-//     own mbarrier with the column's byte count);
+// What bounds it: the chain of column steps (one CTA barrier, one exchange
+// over the cluster each), so what counts is the length of one step in
+// instructions as well as in latencies (here: a warp reduction 56 cycles, a
+// CTA barrier 25, with an OR over the CTA 100, an asynchronous store into
+// another CTA and the wait for it about 600).  An unrolled column loop
+// (column t = register t) made 330 KB of straight-line code, every
+// instruction of it fetched anew in every sub-panel; the rolled form is 85 KB
+// in all.  One 128-column panel, before (unrolled, interchanges in the
+// messages, register FMAs for the trailing columns) and now: m = 128 0.36 ->
+// 0.17 ms, m = 2048 0.354 -> 0.205 ms, m = 8192 0.459 -> 0.325 ms.
+//
+// Pivoting inside a sub-panel is logical: a chosen row is marked done where
+// it is, and every thread tracks the position its rows would have under the
+// reference's interchanges (position j <-> position p_j), which also breaks
+// ties (lowest position: the strict '>' scan of Panel.hpp:52-63).
+//
+// Per column:
+//  1. each warp finds its first maximal |a| (the upper 32 bits of |a| by
+//     redux.sync; the lower bits and the position only on a tie); the lane
+//     that owns the candidate stages it with 1 / pivot in shared memory;
+//  2. after the barrier of the column threads every warp picks the CTA's
+//     candidate from the warps' and the threads store it into every CTA's
+//     shared memory (st.async, 16-byte units, counted in bytes on the
+//     destination's mbarrier for this column; each CTA arms its own mbarrier
+//     with the byte count).  A panel of one CTA skips the exchange;
 //  3. every thread waits (bounded) on its own CTA's mbarrier, picks the winner
-//     from the P messages (first maximal |a|, ties to the lowest row: the
-//     reference's strict '>' scan), the owners of row j and of the winner swap
-//     their register rows through the messages, and every thread scales
-//     (by the sender's 1/pivot, Panel.hpp:78-79) and rank-1 updates its rows
-//     below j (Panel.hpp:80).
+//     from the P messages, scales (by the sender's correctly rounded
+//     1 / pivot, Panel.hpp:78-79), stores the finished column entry to the
+//     shared-memory copy of the sub-panel, and rank-1 updates (Panel.hpp:80).
 // The message buffers alternate between two slots by column parity: a CTA
 // writes slot s for column j + 2 only after it has received every CTA's
 // column j + 1 message, which each CTA sends after all its threads are done
 // with column j's slot, and a CTA re-arms slot s for column j + 2 before it
 // sends column j + 1.  Stopping (an exact zero pivot, seen by every CTA in
 // the same column, or a wait that ran out, which is broadcast to every CTA)
-// is made CTA-uniform at the next __syncthreads_or, and every CTA executes
+// is made CTA-uniform (a lost wait through a shared flag read after the next
+// barrier; slots by column parity, so no thread can see it earlier than
+// another), and every CTA executes
 // the same number of cluster barriers (one per sub-panel, one at the end)
 // whatever happens, so a stop cannot strand a CTA at a barrier.
-// After a sub-panel: the sub-panel is written back, the sub-panel's
-// interchanges are applied to the panel's other columns (ComposePivots,
-// ComposePivots.hpp:81-125, then row moves by the CTA that owns each
-// destination row, all sources read before the cluster barrier), every CTA
-// solves the 16 x (b - c1) block U12 = inv(L11) A12 itself (CTA 0 stores it;
-// L11 is captured from the pivot rows as they arrive), and updates its rows of
-// the remaining panel columns, A[r, c1:b) -= L[r, c0:c1) U12.  The result
-// equals lu::Panel's: the same pivots, and the panel's trailing columns
-// updated in 16-column blocks.  Last, CTA 0 forms inv(unit lower L11) of the
-// panel's top block (16 x 16 diagonal-block inverses, then DMMA doubling).
+// After a sub-panel: every thread writes its rows' entries to their new
+// positions, the interchanges are applied to the panel's other columns (row
+// moves by the CTA that owns each destination row, all sources read before
+// the cluster barrier), every CTA solves the 16 x (b - c1) block
+// U12 = inv(L11) A12 itself (CTA 0 stores it), and updates its rows of the
+// remaining panel columns, A[r, c1:b) -= L[r, c0:c1) U12, with DMMA (L from the
+// shared-memory copy, 32 x 32 warp tiles of C straight from and to L2).  The
+// result equals lu::Panel's: the same pivots, and the panel's trailing columns
+// updated in 16-column blocks.  Last, CTA 0 forms the composed interchanges
+// (ComposePivots.hpp:81-125) from the tracked rows and inv(unit lower L11) of
+// the panel's top block (16 x 16 diagonal-block inverses, then DMMA doubling).
 #include "diag_common.cuh"
 #include "internal.h"
 
@@ -52,37 +68,46 @@ namespace egpu {
 namespace {
 
 constexpr int kRpThreads = 256;
+constexpr int kRpWarps = kRpThreads / 32;  // also the most column warps
 constexpr int kRpW = 16;         // sub-panel width
-constexpr int kRpCandU = 10;     // double2 per candidate: header, 1/pivot, candidate row (8)
-constexpr int kRpMsg = 18;       // double2 per message: a candidate, then row j (8)
+constexpr int kRpMsg = 10;       // double2 per candidate: {|a|, position : row}, {1 / pivot, pivot}, u[0..14]
 constexpr int kRpMaxCl = 16;
-constexpr int kRpNoRow = 0x7fffffff;
+constexpr int kRpNoPos = 0x7fffffff;
+constexpr int kRpLdU = 132;      // 4 mod 16: conflict-free DMMA fragment loads
 
-// shared-memory layout (in doubles)
-constexpr int kRpOffMsg = 0;                                        // [2][kRpMaxCl][kRpMsg] double2
-constexpr int kRpOffCand = kRpOffMsg + 2 * kRpMaxCl * kRpMsg * 2;   // [2][8 warps][kRpCandU] double2 (staging)
-constexpr int kRpOffRowJ = kRpOffCand + 2 * 8 * kRpCandU * 2;       // [2][8] double2 (staging)
-constexpr int kRpOffL11 = kRpOffRowJ + 2 * 8 * 2;                   // 16 x 16 (ld 17)
-constexpr int kRpOffU12 = kRpOffL11 + 16 * 17;                      // [16][128]
-constexpr int kRpOffMv = kRpOffU12 + 16 * 128;                      // [2 * 16][128] row moves
-constexpr int kRpWorkDoubles = kRpOffMv + 2 * kRpW * 128;
+// shared-memory layout (in doubles); the sub-panel copy Lb is [16][R + 4] at the end
+constexpr int kRpOffMsg = 0;                                          // [2][kRpMaxCl][kRpMsg] double2
+constexpr int kRpOffCand = kRpOffMsg + 2 * kRpMaxCl * kRpMsg * 2;     // [2][kRpWarps][kRpMsg] double2
+constexpr int kRpOffL11 = kRpOffCand + 2 * kRpWarps * kRpMsg * 2;     // 16 x 16 (ld 17)
+constexpr int kRpOffU12 = kRpOffL11 + 16 * 17;                        // [16][kRpLdU]
+constexpr int kRpOffMv = kRpOffU12 + 16 * kRpLdU;                     // [2 * 16][128] row moves
+constexpr int kRpOffLb = kRpOffMv + 2 * kRpW * 128;
 constexpr int kRpInvDoubles = 128 * kLDS + 128 + kDiagTmpDoubles;  // the final inv(L11)
-constexpr int kRpSmemDoubles = kRpWorkDoubles > kRpInvDoubles ? kRpWorkDoubles : kRpInvDoubles;
-constexpr uint32_t kRpColBytes(int P) { return (uint32_t)(P * kRpCandU * 16 + 8 * 16); }
-
-// first maximal key over the warp, ties to the lowest row (all lanes get it)
-__device__ __forceinline__ void warp_argmax_key(unsigned long long key, int row, unsigned long long& wkey,
-                                                int& wrow) {
-  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
-  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32) == hi ? (unsigned)key : 0u);
-  wkey = ((unsigned long long)hi << 32) | lo;
-  const unsigned r = __reduce_min_sync(0xffffffffu, key == wkey ? (unsigned)row : (unsigned)kRpNoRow);
-  wrow = (int)r;
+constexpr uint32_t kRpColBytes(int P) { return (uint32_t)(P * kRpMsg * 16); }
+constexpr int rp_smem_doubles(int R) {
+  const int work = kRpOffLb + kRpW * (R + 4) + 32;  // + the last tile's rows past R (read, not stored)
+  return work > kRpInvDoubles ? work : kRpInvDoubles;
 }
 
 // |a| as a key whose unsigned order is the order of |a| (non-negative doubles)
 __device__ __forceinline__ unsigned long long abs_key(double v) {
   return (unsigned long long)__double_as_longlong(fabs(v));
+}
+
+// Lane of the first maximal key over the lanes with pos != kRpNoPos, ties to
+// the lowest position; -1 when no lane takes part.
+__device__ __forceinline__ int warp_argmax(unsigned long long key, int pos) {
+  const bool in = pos != kRpNoPos;
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, in ? hi : 0u);
+  unsigned m = __ballot_sync(0xffffffffu, in && hi == mh);
+  if (__popc(m) > 1) {  // warp-uniform
+    const bool c = in && hi == mh;
+    const unsigned ml = __reduce_max_sync(0xffffffffu, c ? lo : 0u);
+    const unsigned r = __reduce_min_sync(0xffffffffu, c && lo == ml ? (unsigned)pos : (unsigned)kRpNoPos);
+    m = __ballot_sync(0xffffffffu, c && lo == ml && (unsigned)pos == r);
+  }
+  return __ffs(m) - 1;
 }
 
 // 32-bit shared::cluster address of the same object in CTA `rank`
@@ -112,23 +137,30 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
   return ok != 0;
 }
 
+// Barrier of the CT column threads.
+template <int CT>
+__device__ __forceinline__ void column_sync() {
+  asm volatile("barrier.cta.sync 1, %0;" ::"n"(CT) : "memory");
+}
+
 }  // namespace
 
-template <int RT>
+template <int CW, int RT>
 __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b, double* A, long long lda, int* p,
                                                                      int offset, int* image, int* preimage,
-                                                                     double* W, int ldw, DevStatus* st) {
-  constexpr int R = RT * kRpThreads;
-  extern __shared__ double sm[];
+                                                                     double* W, int ldw, DevStatus* st, int R) {
+  constexpr int CT = 32 * CW;  // column threads
+  extern __shared__ __align__(16) double sm[];
   double2* MSG = reinterpret_cast<double2*>(sm + kRpOffMsg);
   double2* CANDB = reinterpret_cast<double2*>(sm + kRpOffCand);
-  double2* ROWJB = reinterpret_cast<double2*>(sm + kRpOffRowJ);
   double* L11 = sm + kRpOffL11;
   double* U12 = sm + kRpOffU12;
   double* MV = sm + kRpOffMv;
-  __shared__ int s_piv[128], s_pre[kRpW];
+  double* Lb = sm + kRpOffLb;  // the sub-panel's finished entries, [16][ldl] by local row
+  const int ldl = R + 4;       // 4 mod 16
+  __shared__ int s_piv[128], s_inv[128];
   __shared__ int s_msrc[2 * kRpW], s_mdst[2 * kRpW];  // the sub-panel's row moves (dst -1: none here)
-  __shared__ int s_skip, s_abort;
+  __shared__ int s_skip, s_abort, s_lost[2];
   __shared__ __align__(8) uint64_t s_bar[2];
 
   const int P = gridDim.x;
@@ -140,9 +172,9 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
   // a failed earlier step: every CTA takes CTA 0's reading of the status
   if (tid == 0) {
     s_skip = (st != nullptr && ((volatile DevStatus*)st)->code != 0);
-    s_abort = 0;
+    s_abort = s_lost[0] = s_lost[1] = 0;
     // one phase per column: this CTA's arrival with the byte count of every
-    // CTA's candidate, plus row j
+    // CTA's candidate
     mbar_init(&s_bar[0], 1);
     mbar_init(&s_bar[1], 1);
     fence_mbar_init();
@@ -159,96 +191,106 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
 
   const int ncols = min(b, m);
   bool stop = false;  // CTA-uniform
-  int lstop = 0;      // this thread saw a zero pivot or a wait that ran out
-  bool abort_sent = false;
-  double v[RT][kRpW];
+  int jdone = 0;      // columns whose pivot is known
+  // the exchange: this thread's units of the CTA's message, by destination
+  constexpr int kSend = (kRpMaxCl * kRpMsg + CT - 1) / CT;
+  uint32_t send_dst[kSend], send_bar[kSend];
+  int send_q[kSend];
+  if (tid < CT)
+#pragma unroll
+    for (int i = 0; i < kSend; ++i) {
+      const int e = tid + i * CT, d = e / kRpMsg, q = e - d * kRpMsg;
+      send_q[i] = d < P ? q : -1;
+      send_dst[i] = d < P ? map_rank(&MSG[(int)cta * kRpMsg + q], (unsigned)d) : 0u;
+      send_bar[i] = d < P ? map_rank(&s_bar[0], (unsigned)d) : 0u;
+    }
+  int gpos = tid;     // where the panel's original row tid (< ncols) is now
   for (int c0 = 0; c0 < ncols; c0 += kRpW) {
     const int c1 = min(ncols, c0 + kRpW), w = c1 - c0;
-    if (!stop) {
-      // ---- load the sub-panel rows into registers (own rows; .cg: no stale L1)
+    int tpos = c0 + (lane & 15);  // where the sub-panel's original row c0 + lane is now (lanes < 16)
+    if (!stop && tid < CT) {
+      // ---- load the sub-panel rows into registers (own rows >= c0; .cg: no stale L1)
+      double v[RT][kRpW];
+      int pos[RT];      // the row's position; kRpNoPos: not a row of the sub-panel
+      bool done[RT];    // already a pivot row
 #pragma unroll
       for (int s = 0; s < RT; ++s) {
-        const int lr = s * kRpThreads + tid;
-#pragma unroll
-        for (int k = 0; k < kRpW; ++k)
-          v[s][k] = (lr < rows && k < w) ? __ldcg(&A[(long long)(c0 + k) * lda + r0 + lr]) : 0.0;
+        const int lr = s * CT + tid;
+        const bool act = lr < rows && r0 + lr >= c0;
+        pos[s] = act ? r0 + lr : kRpNoPos;
+        done[s] = !act;
       }
-      // ---- column loop (unrolled: column t of the sub-panel is register t)
+      {
+        const double* src = A + (long long)c0 * lda + r0 + tid;
 #pragma unroll
-      for (int t = 0; t < kRpW; ++t) {
-        if (t >= w) break;
+        for (int k = 0; k < kRpW; ++k) {
+#pragma unroll
+          for (int s = 0; s < RT; ++s) v[s][k] = (!done[s] && k < w) ? __ldcg(src + s * CT) : 0.0;
+          src += lda;
+        }
+      }
+      bool stop_after = false;  // this warp lost a wait
+      // ---- column loop
+#pragma unroll 1
+      for (int t = 0; t < w; ++t) {
         const int j = c0 + t, par = j & 1;
         const uint32_t phase = (uint32_t)(j >> 1) & 1u;
-        double2* CAND = CANDB + par * 8 * kRpCandU;
-        double2* ROWJ = ROWJB + par * 8;
-        // 1. warp candidate; its owner stages the row and 1/pivot
+        double2* CAND = CANDB + par * kRpWarps * kRpMsg;
+        // 1. the warp's candidate; its owner stages it
         unsigned long long key = 0ull;
-        int krow = kRpNoRow;
+        int kpos = kRpNoPos, ks = 0;
+        double pv0 = 1.0;
 #pragma unroll
-        for (int s = 0; s < RT; ++s) {
-          const int lr = s * kRpThreads + tid, r = r0 + lr;
-          if (lr < rows && r >= j) {
-            const unsigned long long kk = abs_key(v[s][t]);
-            if (krow == kRpNoRow || kk > key) { key = kk; krow = r; }  // slots ascend in row
-          }
+        for (int s = 0; s < RT; ++s) {  // branch-free: a row that is done counts as |a| = 0 at no position
+          const unsigned long long kk = done[s] ? 0ull : abs_key(v[s][0]);
+          const int kp = done[s] ? kRpNoPos : pos[s];
+          const bool better = kk > key || (kk == key && kp < kpos);
+          key = better ? kk : key;
+          kpos = better ? kp : kpos;
+          ks = better ? s : ks;
+          pv0 = better ? v[s][0] : pv0;
         }
-        unsigned long long wkey;
-        int wrow;
-        warp_argmax_key(key, krow, wkey, wrow);
-        double2* cw = &CAND[warp * kRpCandU];
-        if (wrow == kRpNoRow) {
-          if (lane == 0) cw[0] = make_double2(0.0, (double)kRpNoRow);
-        } else {
+        const double pinv = __drcp_rn(pv0);  // the correctly rounded 1 / pivot
+        const int wl = warp_argmax(key, kpos);
+        double2* cw = &CAND[warp * kRpMsg];
+        if (wl < 0) {
+          if (lane == 0) cw[0] = make_double2(0.0, __hiloint2double(kRpNoPos, 0));
+        } else if (lane == wl) {
+          cw[0] = make_double2(__longlong_as_double((long long)key),
+                               __hiloint2double(kpos, r0 + ks * CT + tid));
+          cw[1] = make_double2(pinv, pv0);
 #pragma unroll
           for (int s = 0; s < RT; ++s)
-            if (r0 + s * kRpThreads + tid == wrow) {
-              cw[0] = make_double2(__longlong_as_double((long long)wkey), (double)wrow);
-              cw[1] = make_double2(__drcp_rn(v[s][t]), 0.0);  // the correctly rounded 1 / pivot
+            if (s == ks) {
 #pragma unroll
-              for (int q = 0; q < 8; ++q) cw[2 + q] = make_double2(v[s][2 * q], v[s][2 * q + 1]);
+              for (int q = 0; q < 8; ++q)
+                cw[2 + q] = make_double2(v[s][2 * q + 1], q < 7 ? v[s][2 * q + 2] : 0.0);
             }
         }
-        // row j's owner stages it for the message
-        const bool ownj = j >= r0 && j < r0 + rows;
-        if (ownj && ((j - r0) & (kRpThreads - 1)) == tid) {
-          const int sj = (j - r0) / kRpThreads;
+        column_sync<CT>();
+        // a wait of this CTA that ran out in the last column (written before
+        // this barrier; the slot of this column is another one)
+        const int lost = *(volatile int*)&s_lost[par ^ 1];
+        // 2. the CTA's candidate, sent to every CTA
+        const double2* cand;  // the P (or CW) candidates to choose the winner from
+        int wc;
+        if (P > 1) {
+          {
+            unsigned long long ck = 0ull;
+            int cpos = kRpNoPos;
+            if (lane < CW) {
+              const double2 h = CAND[lane * kRpMsg];
+              ck = (unsigned long long)__double_as_longlong(h.x);
+              cpos = __double2hiint(h.y);
+            }
+            const int wsrc = max(0, warp_argmax(ck, cpos));
 #pragma unroll
-          for (int s = 0; s < RT; ++s)
-            if (s == sj)
-#pragma unroll
-              for (int q = 0; q < 8; ++q) ROWJ[q] = make_double2(v[s][2 * q], v[s][2 * q + 1]);
-        }
-        if (__syncthreads_or(lstop)) {
-          stop = true;
-          break;
-        }
-        // 2. CTA candidate; lane L of warps 0-1 stores units L%4, L%4 + 4, ...
-        //    of the message into CTA L/4 (asynchronous stores counted on that
-        //    CTA's mbarrier for this column)
-        if (warp < 2) {
-          unsigned long long ck = 0ull;
-          int crow = kRpNoRow;
-          if (lane < 8) {
-            const double2 h = CAND[lane * kRpCandU];
-            ck = (unsigned long long)__double_as_longlong(h.x);
-            crow = (int)h.y;
+            for (int i = 0; i < kSend; ++i)
+              if (send_q[i] >= 0)
+                st_async(send_dst[i] + (uint32_t)(par * kRpMaxCl * kRpMsg * 16), CAND[wsrc * kRpMsg + send_q[i]],
+                         send_bar[i] + 8u * (uint32_t)par);
           }
-          unsigned long long bk;
-          int brow;
-          warp_argmax_key(ck, crow, bk, brow);
-          const unsigned cwm = __ballot_sync(0xffffffffu, lane < 8 && crow == brow && ck == bk);
-          const int wsrc = cwm ? __ffs(cwm) - 1 : 0;
-          const int nunits = ownj ? kRpMsg : kRpCandU;
-          const int L = warp * 32 + lane, d = L >> 2;
-          if (d < P) {
-            const uint32_t dst = map_rank(&MSG[(par * kRpMaxCl + (int)cta) * kRpMsg], (unsigned)d);
-            const uint32_t bar = map_rank(&s_bar[par], (unsigned)d);
-            for (int u = L & 3; u < nunits; u += 4)
-              st_async(dst + 16u * (uint32_t)u, u < kRpCandU ? CAND[wsrc * kRpCandU + u] : ROWJ[u - kRpCandU], bar);
-          }
-        }
-        // 3. every CTA's message (bounded wait; a wait that runs out stops the cluster)
-        {
+          // 3. every CTA's message (bounded wait; a wait that runs out stops the cluster)
           bool got = false;
           for (long long it = 0; it < kSpinLimit; ++it) {
             if (mbar_try_wait_cluster(&s_bar[par], phase)) {
@@ -262,252 +304,262 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
           // before every CTA has sent column j + 1, which this CTA does after this
           if (got && tid == 0) mbar_expect_tx(&s_bar[par], kRpColBytes(P));
           if (!got) {
-            lstop = 1;
-            if (!abort_sent) {
-              abort_sent = true;
-              set_status(st, kTimeout, 41);
-              for (int d = 0; d < P; ++d) st_cluster(map_rank(&s_abort, (unsigned)d), 1);
-            }
+            s_lost[par] = 1;
+            set_status(st, kTimeout, 41);
+            for (int d = 0; d < P; ++d) st_cluster(map_rank(&s_abort, (unsigned)d), 1);
           }
+          // the warp goes on together: one lane's lost wait ends the column for all
+          if (__any_sync(0xffffffffu, !got || lost)) {
+            if (lost) {  // CTA-uniform: known to every column thread since the barrier
+              stop = true;
+              break;
+            }
+            stop_after = true;
+            continue;
+          }
+          cand = MSG + par * kRpMaxCl * kRpMsg;
+        } else {
+          cand = CAND;
         }
-        if (!lstop) {
-          // winner over the P messages (first maximal |a|, lowest row on ties)
+        // the winner (first maximal |a|, lowest position on ties)
+        {
           unsigned long long gk = 0ull;
-          int grow = kRpNoRow;
-          if (lane < P) {
-            const double2 h = MSG[(par * kRpMaxCl + lane) * kRpMsg];
+          int gp = kRpNoPos;
+          if (lane < (P > 1 ? P : CW)) {
+            const double2 h = cand[lane * kRpMsg];
             gk = (unsigned long long)__double_as_longlong(h.x);
-            grow = (int)h.y;
+            gp = __double2hiint(h.y);
           }
-          unsigned long long wk;
-          int wr;
-          warp_argmax_key(gk, grow, wk, wr);
-          const unsigned cm = __ballot_sync(0xffffffffu, lane < P && grow == wr && gk == wk);
-          const int wc = cm ? __ffs(cm) - 1 : 0;
-          const double2* wm = &MSG[(par * kRpMaxCl + wc) * kRpMsg];
-          const double2* wmsg = wm + 2;                                               // winner row
-          const double2* jmsg = &MSG[(par * kRpMaxCl + j / R) * kRpMsg + kRpCandU];   // row j
-          const double2 pv = wmsg[t / 2];
-          const double wv = (t & 1) ? pv.y : pv.x;  // the pivot
-          if (wr == kRpNoRow || wv == 0.0) {  // exact zero pivot: SingularMatrixException (Panel.hpp:76-77)
-            if (cta == 0 && tid == 0) set_status(st, kSingular, offset + j + 1);
-            lstop = 1;
+          wc = warp_argmax(gk, gp);
+        }
+        const double2* wm = cand + max(wc, 0) * kRpMsg;
+        const double whd = wm[0].y;
+        const int wpos = __double2hiint(whd), wrow = __double2loint(whd);
+        const double2 wi = wm[1];
+        if (wc < 0 || wi.y == 0.0) {  // exact zero pivot: SingularMatrixException (Panel.hpp:76-77)
+          if (cta == 0 && tid == 0) set_status(st, kSingular, offset + j + 1);
+          stop = true;  // the same messages in every CTA: cluster-uniform
+          break;
+        }
+        jdone = j + 1;
+        if (tid == 0) {
+          s_piv[j] = wpos;
+          s_msrc[kRpW + t] = wrow;
+        }
+        // interchange of positions j and wpos (Panel.hpp:66-72)
+        if (tpos == j) tpos = wpos;
+        else if (tpos == wpos) tpos = j;
+        if (gpos == j) gpos = wpos;
+        else if (gpos == wpos) gpos = j;
+        double u[kRpW];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const double2 x = wm[2 + q];
+          u[2 * q] = x.x;
+          u[2 * q + 1] = x.y;
+        }
+        // the winner's row is final: its entries go to the copy as they are
+#pragma unroll
+        for (int s = 0; s < RT; ++s) {
+          const int lr = s * CT + tid;
+          if (pos[s] == j) pos[s] = wpos;
+          if (r0 + lr == wrow && pos[s] != kRpNoPos) {
+            pos[s] = j;
+            done[s] = true;
+#pragma unroll
+            for (int k = 0; k < kRpW; ++k)
+              if (t + k < kRpW) Lb[(t + k) * ldl + lr] = v[s][k];
+          }
+        }
+        // scale (Panel.hpp:78-79) and rank-1 update (Geru, :80); what rows
+        // that are done (or no rows) compute here is not used
+#pragma unroll
+        for (int s = 0; s < RT; ++s) {
+          const double l = v[s][0] * wi.x;
+          if (!done[s]) Lb[t * ldl + s * CT + tid] = l;
+#pragma unroll
+          for (int k = 0; k < kRpW - 1; ++k) v[s][k] = fma(-l, u[k], v[s][k + 1]);
+          v[s][kRpW - 1] = 0.0;
+        }
+      }
+      stop = stop || stop_after;
+      if (!stop) {
+        // ---- write the sub-panel back, every row to its new position
+#pragma unroll
+        for (int s = 0; s < RT; ++s) {
+          if (pos[s] != kRpNoPos) {
+            double* dst = A + (long long)c0 * lda + pos[s];
+            const double* from = Lb + s * CT + tid;
+#pragma unroll 4
+            for (int k = 0; k < w; ++k) dst[k * lda] = from[k * ldl];
+          }
+        }
+        // The sub-panel's row moves: move i takes row c0 + i to where it is
+        // now; move 16 + i takes the row chosen as pivot i to c0 + i when it
+        // came from below the sub-panel.  A move is kept when this CTA owns
+        // its destination.
+        if (warp == 0) {
+          __syncwarp();  // lane 0's s_msrc
+          const int i = lane & 15;
+          if (lane < kRpW) {
+            s_msrc[i] = c0 + i;
+            s_mdst[i] = (i < w && tpos != c0 + i && tpos >= r0 && tpos < r0 + rows) ? tpos : -1;
           } else {
-            if (tid == 0) s_piv[j] = wr;
-            if (cta == 0 && tid == 0) p[j] = wr + offset;
-            // the pivot row is final: its entries left of t are row t of L11
-            if (tid == 32) {
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const double2 x = wmsg[q];
-                if (2 * q < t) L11[t + (2 * q) * 17] = x.x;
-                if (2 * q + 1 < t) L11[t + (2 * q + 1) * 17] = x.y;
-              }
-            }
-            // row interchange inside the sub-panel (Panel.hpp:66-72)
-            if (wr != j) {
-#pragma unroll
-              for (int s = 0; s < RT; ++s) {
-                const int r = r0 + s * kRpThreads + tid;
-                if (r == j) {
-#pragma unroll
-                  for (int q = 0; q < 8; ++q) { const double2 x = wmsg[q]; v[s][2 * q] = x.x; v[s][2 * q + 1] = x.y; }
-                } else if (r == wr) {
-#pragma unroll
-                  for (int q = 0; q < 8; ++q) { const double2 x = jmsg[q]; v[s][2 * q] = x.x; v[s][2 * q + 1] = x.y; }
-                }
-              }
-            }
-            double u[kRpW];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const double2 x = wmsg[q];
-              u[2 * q] = x.x;
-              u[2 * q + 1] = x.y;
-            }
-            // scale (Panel.hpp:78-79) and rank-1 update (Geru, :80) of own rows > j
-            const double inv = wm[1].x;
-#pragma unroll
-            for (int s = 0; s < RT; ++s) {
-              const int lr = s * kRpThreads + tid, r = r0 + lr;
-              if (lr < rows && r > j) {
-                const double l = v[s][t] * inv;
-                v[s][t] = l;
-#pragma unroll
-                for (int k = t + 1; k < kRpW; ++k) v[s][k] = fma(-l, u[k], v[s][k]);
-              }
-            }
+            const int d = c0 + i;
+            s_mdst[kRpW + i] = (i < w && s_msrc[kRpW + i] >= c1 && d >= r0 && d < r0 + rows) ? d : -1;
           }
         }
       }
     }
-    stop = __syncthreads_or(stop || lstop);
-    if (!stop) {
-      // ---- write the sub-panel back (own rows)
-#pragma unroll
-      for (int s = 0; s < RT; ++s) {
-        const int lr = s * kRpThreads + tid;
-        if (lr < rows)
-#pragma unroll
-          for (int k = 0; k < kRpW; ++k)
-            if (k < w) A[(long long)(c0 + k) * lda + r0 + lr] = v[s][k];
-      }
-    }
-    // ---- ComposePivots (ComposePivots.hpp:81-125) of the sub-panel, relative
-    // to row c0, and the row moves it implies: move i takes row c0+i to
-    // c0+img[i]; move w+i takes row c0+pre[i] to c0+i when pre[i] >= w (a row
-    // from below the sub-panel).  A move is kept when this CTA owns its
-    // destination.
-    if (!stop && tid < w) {
-      const int i = tid;
-      int k = s_piv[c0 + i] - c0;
-      for (int q = i - 1; q >= 0; --q) {
-        const int pq = s_piv[c0 + q] - c0;
-        if (pq == k) k = q;
-        else if (q == k) k = pq;
-      }
-      const int pre = k;
-      k = i;
-      for (int q = 0; q < min(k + 1, w); ++q) {
-        const int pq = s_piv[c0 + q] - c0;
-        if (pq == k) k = q;
-        else if (q == k) k = pq;
-      }
-      const int img = k;
-      s_pre[i] = pre;
-      int src = c0 + i, d = c0 + img;
-      s_msrc[i] = src;
-      s_mdst[i] = (d != src && d >= r0 && d < r0 + rows) ? d : -1;
-      src = c0 + pre;
-      d = c0 + i;
-      s_msrc[w + i] = src;
-      s_mdst[w + i] = (pre >= w && d != src && d >= r0 && d < r0 + rows) ? d : -1;
-    }
-    __syncthreads();
+    stop = __syncthreads_or(stop);
     // The moves apply to the panel's other columns [0, c0) and [c1, b); rows
     // c0..c1-1 of columns [c1, b) become U12 and are not moved; U12's input
-    // row i is the old row c0+pre[i].
+    // row i is the old row of pivot i.
     const int nout = b - w;
     const int ntr = b - c1;  // trailing panel columns
+    constexpr int kMvPer = 2 * kRpW * 128 / kRpThreads, kU12Per = kRpW * 128 / kRpThreads;
+    const int mcol = tid & 127, mq = tid >> 7;  // this thread's column and first move of the moves
     if (!stop) {
       // all of a thread's gathers are issued before any is stored, so their
       // L2 latencies overlap
-      const int cc = tid & 127;
-      double g[kRpW];
+      double g[kMvPer], gu[kU12Per];
 #pragma unroll
-      for (int q = 0; q < kRpW; ++q) {
-        const int mv = 2 * q + (tid >> 7);
-        const int d = mv < 2 * w ? s_mdst[mv] : -1;
+      for (int q = 0; q < kMvPer; ++q) {
+        const int mv = q * (kRpThreads / 128) + mq, d = s_mdst[mv];
         g[q] = 0.0;
-        if (d >= 0 && cc < nout) {
-          const int col = cc < c0 ? cc : cc + w;
+        if (d >= 0 && mcol < nout) {
+          const int col = mcol < c0 ? mcol : mcol + w;
           if (!(col >= c1 && d < c1)) g[q] = __ldcg(&A[(long long)col * lda + s_msrc[mv]]);
         }
       }
-      double gu[kRpW * 128 / kRpThreads];
 #pragma unroll
-      for (int q = 0; q < kRpW * 128 / kRpThreads; ++q) {
-        const int idx = tid + q * kRpThreads, i = idx >> 7, c = idx & 127;
-        gu[q] = (i < w && c < ntr) ? __ldcg(&A[(long long)(c1 + c) * lda + c0 + s_pre[i]]) : 0.0;
+      for (int q = 0; q < kU12Per; ++q) {
+        const int i = q * (kRpThreads / 128) + mq;
+        gu[q] = (i < w && mcol < ntr) ? __ldcg(&A[(long long)(c1 + mcol) * lda + s_msrc[kRpW + i]]) : 0.0;
       }
 #pragma unroll
-      for (int q = 0; q < kRpW; ++q) {
-        const int mv = 2 * q + (tid >> 7);
-        const int d = mv < 2 * w ? s_mdst[mv] : -1;
-        if (d >= 0 && cc < nout) {
-          const int col = cc < c0 ? cc : cc + w;
-          if (!(col >= c1 && d < c1)) MV[mv * 128 + cc] = g[q];
-        }
-      }
+      for (int q = 0; q < kMvPer; ++q) MV[(q * (kRpThreads / 128) + mq) * 128 + mcol] = g[q];
 #pragma unroll
-      for (int q = 0; q < kRpW * 128 / kRpThreads; ++q) {
-        const int idx = tid + q * kRpThreads, i = idx >> 7, c = idx & 127;
-        if (i < w && c < ntr) U12[i * 128 + c] = gu[q];
+      for (int q = 0; q < kU12Per; ++q) {
+        const int i = q * (kRpThreads / 128) + mq;
+        if (i < w && mcol < ntr) U12[i * kRpLdU + mcol] = gu[q];
       }
     }
-    // every source read (and CTA 0's sub-panel written) cluster-wide
+    // every source read and every sub-panel row written, cluster-wide
     cluster_arrive_release();
     cluster_wait_acquire();
     if (!stop) {
-      const int cc = tid & 127;
-      for (int mv = tid >> 7; mv < 2 * w; mv += 2) {
-        const int d = s_mdst[mv];
-        if (d >= 0 && cc < nout) {
-          const int col = cc < c0 ? cc : cc + w;
-          if (!(col >= c1 && d < c1)) A[(long long)col * lda + d] = MV[mv * 128 + cc];
+#pragma unroll
+      for (int q = 0; q < kMvPer; ++q) {
+        const int mv = q * (kRpThreads / 128) + mq, d = s_mdst[mv];
+        if (d >= 0 && mcol < nout) {
+          const int col = mcol < c0 ? mcol : mcol + w;
+          if (!(col >= c1 && d < c1)) A[(long long)col * lda + d] = MV[mv * 128 + mcol];
         }
+      }
+      if (ntr > 0) {  // a trailing block follows only a full sub-panel: w = 16
+        // L11 from the pivot rows, and the shared-memory copy of the rows that
+        // were moved into this CTA's part
+        const int i = tid >> 4, k = tid & 15, d = s_mdst[i];
+        const double x = __ldcg(&A[(long long)(c0 + k) * lda + c0 + i]);
+        if (d >= c1) Lb[k * ldl + d - r0] = __ldcg(&A[(long long)(c0 + k) * lda + d]);
+        L11[i + k * 17] = x;
       }
     }
     __syncthreads();
     if (!stop && ntr > 0) {
       // U12 := inv(unit lower L11) A12, one column per thread, in shared memory
-      for (int cc = tid; cc < ntr; cc += kRpThreads) {
+      if (tid < ntr) {
         double u[kRpW];
 #pragma unroll
-        for (int i = 0; i < kRpW; ++i) u[i] = (i < w) ? U12[i * 128 + cc] : 0.0;
+        for (int i = 0; i < kRpW; ++i) u[i] = U12[i * kRpLdU + tid];
 #pragma unroll
-        for (int i = 1; i < kRpW; ++i) {
-          double x = u[i];
+        for (int i = 0; i < kRpW - 1; ++i)
 #pragma unroll
-          for (int k = 0; k < kRpW; ++k)
-            if (k < i && i < w) x = fma(-L11[i + k * 17], u[k], x);
-          u[i] = x;
-        }
+          for (int k = i + 1; k < kRpW; ++k) u[k] = fma(-L11[k + i * 17], u[i], u[k]);
 #pragma unroll
-        for (int i = 0; i < kRpW; ++i)
-          if (i < w) {
-            U12[i * 128 + cc] = u[i];
-            if (cta == 0) A[(long long)(c1 + cc) * lda + c0 + i] = u[i];
-          }
+        for (int i = 0; i < kRpW; ++i) U12[i * kRpLdU + tid] = u[i];
+        if (cta == 0)
+#pragma unroll
+          for (int i = 0; i < kRpW; ++i) A[(long long)(c1 + tid) * lda + c0 + i] = u[i];
+      } else if (tid < 128) {
+#pragma unroll
+        for (int i = 0; i < kRpW; ++i) U12[i * kRpLdU + tid] = 0.0;
       }
     }
     __syncthreads();
     if (!stop && ntr > 0) {
-      // A[r, c1:b) -= L[r, c0:c1) U12 for own rows r >= c1 (L in registers),
-      // kB columns at a time, the next batch's loads in flight while the
-      // current one is updated
-      constexpr int kB = RT >= 4 ? 4 : 8;
-      double xa[RT][kB], xb[RT][kB];
-      auto load = [&](double (&x)[RT][kB], int cb) {
-#pragma unroll
-        for (int s = 0; s < RT; ++s) {
-          const int lr = s * kRpThreads + tid, r = r0 + lr;
-#pragma unroll
-          for (int q = 0; q < kB; ++q)
-            x[s][q] = (lr < rows && r >= c1 && cb + q < ntr) ? __ldcg(&A[(long long)(c1 + cb + q) * lda + r]) : 0.0;
-        }
+      // A[r, c1:b) -= L[r, c0:c1) U12 for own rows r >= c1: 32 x 32 warp tiles
+      const int lr1 = max(0, c1 - r0);  // a multiple of 16
+      const int g = lane >> 2, t4 = lane & 3;
+      const int trow = (rows - lr1 + 31) / 32, tcol = (ntr + 31) / 32;
+      const int ntile = trow * tcol;
+      auto row_col = [&](int tile, int& lr, int& cb) {
+        lr = lr1 + (tile % trow) * 32;
+        cb = (tile / trow) * 32;
       };
-      auto update = [&](double (&x)[RT][kB], int cb) {
-        // U12 pairs as 16-byte shared loads (cb is even): one load feeds 2 RT FMAs
+      // element (i, jn, q) of a tile: row 16 i + g (+ 8), column 8 jn + 2 t4 (+ 1)
+      auto load = [&](double (&acc)[2][4][4], int tile) {
+        int lr, cb;
+        row_col(tile, lr, cb);
+        const double* C = A + (long long)(c1 + cb + 2 * t4) * lda + r0 + lr + g;
 #pragma unroll
-        for (int k = 0; k < kRpW; ++k) {
-          if (k < w) {
-            double2 uu[kB / 2];
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int h = 0; h < kB / 2; ++h) uu[h] = *reinterpret_cast<const double2*>(&U12[k * 128 + cb + 2 * h]);
+          for (int jn = 0; jn < 4; ++jn)
 #pragma unroll
-            for (int q = 0; q < kB; ++q) {
-              const double u = (q & 1) ? uu[q / 2].y : uu[q / 2].x;
-#pragma unroll
-              for (int s = 0; s < RT; ++s) x[s][q] = fma(-v[s][k], u, x[s][q]);
+            for (int q = 0; q < 4; ++q) {
+              const int rr = 16 * i + ((q >= 2) ? 8 : 0), cc = 8 * jn + (q & 1);
+              acc[i][jn][q] =
+                  (lr + g + rr < rows && cb + 2 * t4 + cc < ntr) ? __ldcg(&C[(long long)cc * lda + rr]) : 0.0;
             }
-          }
-        }
-#pragma unroll
-        for (int s = 0; s < RT; ++s) {
-          const int lr = s * kRpThreads + tid, r = r0 + lr;
-#pragma unroll
-          for (int q = 0; q < kB; ++q)
-            if (lr < rows && r >= c1 && cb + q < ntr) A[(long long)(c1 + cb + q) * lda + r] = x[s][q];
-        }
       };
-      load(xa, 0);
-      for (int cb = 0; cb < ntr; cb += 2 * kB) {
-        if (cb + kB < ntr) load(xb, cb + kB);
-        update(xa, cb);
-        if (cb + kB < ntr) {
-          if (cb + 2 * kB < ntr) load(xa, cb + 2 * kB);
-          update(xb, cb + kB);
+      auto update = [&](double (&acc)[2][4][4], int tile) {
+        int lr, cb;
+        row_col(tile, lr, cb);
+#pragma unroll
+        for (int k0 = 0; k0 < kRpW; k0 += 8) {
+          double af[2][4], bf[4][2];
+          const double* la = &Lb[(k0 + t4) * ldl + lr + g];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {  // rows past the CTA's end are computed and not stored
+            af[i][0] = -la[16 * i];
+            af[i][1] = -la[16 * i + 8];
+            af[i][2] = -la[4 * ldl + 16 * i];
+            af[i][3] = -la[4 * ldl + 16 * i + 8];
+          }
+          const double* ub = &U12[(k0 + t4) * kRpLdU + cb + g];
+#pragma unroll
+          for (int jn = 0; jn < 4; ++jn) {
+            bf[jn][0] = ub[8 * jn];
+            bf[jn][1] = ub[4 * kRpLdU + 8 * jn];
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int jn = 0; jn < 4; ++jn) dmma_16x8x8(acc[i][jn], af[i], bf[jn]);
+        }
+        double* C = A + (long long)(c1 + cb + 2 * t4) * lda + r0 + lr + g;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int jn = 0; jn < 4; ++jn)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int rr = 16 * i + ((q >= 2) ? 8 : 0), cc = 8 * jn + (q & 1);
+              if (lr + g + rr < rows && cb + 2 * t4 + cc < ntr) C[(long long)cc * lda + rr] = acc[i][jn][q];
+            }
+      };
+      // the next tile's loads are in flight while the current one is updated
+      double xa[2][4][4], xb[2][4][4];
+      if (warp < ntile) load(xa, warp);
+#pragma unroll 1
+      for (int tile = warp; tile < ntile; tile += 2 * kRpWarps) {
+        if (tile + kRpWarps < ntile) load(xb, tile + kRpWarps);
+        update(xa, tile);
+        if (tile + kRpWarps < ntile) {
+          if (tile + 2 * kRpWarps < ntile) load(xa, tile + 2 * kRpWarps);
+          update(xb, tile + kRpWarps);
         }
       }
     }
@@ -516,28 +568,23 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
   // all CTAs done with each other's shared memory and with the panel
   cluster_arrive_release();
   cluster_wait_acquire();
+  if (cta != 0) return;
+  if (tid < jdone) p[tid] = s_piv[tid] + offset;
   if (stop) return;
-  if (cta == 0 && tid < ncols) {  // ComposePivots over the whole panel
-    const int i = tid;
-    int k = s_piv[i];
-    for (int q = i - 1; q >= 0; --q) {
-      const int pq = s_piv[q];
-      if (pq == k) k = q;
-      else if (q == k) k = pq;
-    }
-    preimage[i] = k;
-    k = i;
-    for (int q = 0; q < min(k + 1, ncols); ++q) {
-      const int pq = s_piv[q];
-      if (pq == k) k = q;
-      else if (q == k) k = pq;
-    }
-    image[i] = k;
+  // ComposePivots (ComposePivots.hpp:81-125) over the whole panel: original
+  // row i is now at gpos; position i holds the original row that is there now,
+  // or the row its pivot was first taken from
+  if (tid < 128) s_inv[tid] = -1;
+  __syncthreads();
+  if (tid < ncols) {
+    image[tid] = gpos;
+    if (gpos < ncols) s_inv[gpos] = tid;
   }
+  __syncthreads();
+  if (tid < ncols) preimage[tid] = s_inv[tid] >= 0 ? s_inv[tid] : s_piv[tid];
   if (W == nullptr) return;
   // inv(unit lower L11) of the panel's top bb x bb block, by CTA 0: 16 x 16
   // diagonal-block inverses by warps, then the DMMA doubling steps
-  if (cta != 0) return;
   const int bb = ncols;
   double* S = sm;
   for (int e0 = tid; e0 < bb * bb; e0 += 8 * kRpThreads) {  // .cg: rows written by other CTAs
@@ -567,51 +614,64 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
   }
 }
 
-// Launch the register-resident panel when m fits one cluster (m <= 16 * 1024
-// rows with a 16-CTA cluster) and b <= 128.  Returns EGPU_ERR_UNSUPPORTED when it does not apply.
+// Launch the register-resident panel when m fits one cluster (b <= m <= 16 x
+// 1024 rows with a 16-CTA cluster) and b <= 128.  Returns EGPU_ERR_UNSUPPORTED
+// when it does not apply.  The fewest rows per CTA that fit one cluster: the
+// trailing updates inside the panel get shorter with every CTA (m = 2048:
+// 0.248 ms with 128 rows a CTA, 0.268 with 256, 0.327 with 512, measured on an
+// earlier form of the kernel), the exchange only a little longer.  Four
+// column warps up to 256 rows a CTA and eight above: four warps with four
+// rows a thread measured 0.36 ms at m = 8192 against 0.34 for eight with two.
 int launch_lu_panel_rp(cudaStream_t st, int m, int b, double* A, long long lda, int* p, int offset, int* image,
                        int* preimage, double* W, int ldw, DevStatus* status, int cluster_max) {
-  if (b > 128 || b < 1 || cluster_max < 1) return EGPU_ERR_UNSUPPORTED;
-  const size_t smem = sizeof(double) * kRpSmemDoubles;
-  static int cl_max[3] = {-1, -1, -1};  // per RT: largest cluster the kernel can be scheduled with
-  auto kern_of = [](int rt) {
-    return rt == 1 ? lu_panel_rp_kernel<1> : (rt == 2 ? lu_panel_rp_kernel<2> : lu_panel_rp_kernel<4>);
+  if (b > 128 || b < 1 || m < b || cluster_max < 1) return EGPU_ERR_UNSUPPORTED;
+  using Kern = void (*)(int, int, double*, long long, int*, int, int*, int*, double*, int, DevStatus*, int);
+  struct Config {
+    Kern kern;
+    int rmax;    // rows per CTA
+    int cl_max;  // largest cluster it can be scheduled with (-1: not asked yet)
   };
-  int RT = 0, P = 0;
-  for (int ai = 0; ai < 3 && RT == 0; ++ai) {  // fewest rows per thread that fit one cluster
-    const int rt = 1 << ai;
-    if (cl_max[ai] < 0) {
-      cl_max[ai] = 0;
-      auto kern = kern_of(rt);
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-          cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-        for (int c : {16, 8}) {
+  static Config configs[4] = {{lu_panel_rp_kernel<4, 1>, 128, -1}, {lu_panel_rp_kernel<4, 2>, 256, -1},
+                              {lu_panel_rp_kernel<8, 2>, 512, -1}, {lu_panel_rp_kernel<8, 4>, 1024, -1}};
+  Kern kern = nullptr;
+  size_t smem = 0;
+  int P = 0, R = 0;
+  for (Config& c : configs) {  // the fewest rows per CTA that fit one cluster
+    smem = sizeof(double) * rp_smem_doubles(c.rmax);
+    if (c.cl_max < 0) {
+      int fits = 0;
+      if (cudaFuncSetAttribute(c.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+          cudaFuncSetAttribute(c.kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        for (int n : {16, 8}) {
           cudaLaunchConfig_t cfg = {};
-          cfg.gridDim = dim3(c);
+          cfg.gridDim = dim3(n);
           cfg.blockDim = dim3(kRpThreads);
           cfg.dynamicSmemBytes = smem;
           cudaLaunchAttribute attr[1];
           attr[0].id = cudaLaunchAttributeClusterDimension;
-          attr[0].val.clusterDim.x = c;
+          attr[0].val.clusterDim.x = n;
           attr[0].val.clusterDim.y = 1;
           attr[0].val.clusterDim.z = 1;
           cfg.attrs = attr;
           cfg.numAttrs = 1;
           int ncl = 0;
-          if (cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg) == cudaSuccess && ncl > 0) {
-            cl_max[ai] = c;
+          if (cudaOccupancyMaxActiveClusters(&ncl, c.kern, &cfg) == cudaSuccess && ncl > 0) {
+            fits = n;
             break;
           }
         }
       }
       cudaGetLastError();
+      c.cl_max = fits;
     }
-    const int cmax = std::min(cl_max[ai], cluster_max > 0 ? kRpMaxCl : 0);
-    const int pp = (m + rt * kRpThreads - 1) / (rt * kRpThreads);
-    if (cmax > 0 && pp <= cmax) { RT = rt; P = pp; }
+    const int cmax = std::min(std::min(c.cl_max, kRpMaxCl), cluster_max);
+    if (cmax < 1 || (m + c.rmax - 1) / c.rmax > cmax) continue;
+    kern = c.kern;
+    R = std::max(128, ((m + cmax - 1) / cmax + 15) / 16 * 16);
+    P = (m + R - 1) / R;
+    break;
   }
-  if (RT == 0) return EGPU_ERR_UNSUPPORTED;
-  auto kern = kern_of(RT);
+  if (kern == nullptr) return EGPU_ERR_UNSUPPORTED;
   TraceMark tm(st, kTracePanel, (double)m * b * b, 16.0 * m * b);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(P);
@@ -625,7 +685,7 @@ int launch_lu_panel_rp(cudaStream_t st, int m, int b, double* A, long long lda, 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, m, b, A, lda, p, offset, image, preimage, W, ldw, status);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, m, b, A, lda, p, offset, image, preimage, W, ldw, status, R);
   count_launch();
   if (e != cudaSuccess) {
     set_last_error(e, "lu_panel_rp launch", __FILE__, __LINE__);

@@ -196,18 +196,28 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const SmallParams p) {
   // every load of the CTA is done before any store (C may alias A or B)
   __syncthreads();
   if (!live) return;
+  // all of the tile's C loads in flight before the first is used
+  double cc[2][4][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const int m = row0 + 16 * i + g + (r >= 2 ? 8 : 0);
-        const int n = col0 + 8 * j + 2 * t + (r & 1);
-        if (m >= p.M || n >= p.N) continue;
-        if ((p.tri == 1 && m < n) || (p.tri == 2 && m > n)) continue;
-        double* c = &p.C[m + (long long)n * p.ldc];
-        *c = p.beta == 0.0 ? p.alpha * acc[i][j][r] : fma(p.beta, *c, p.alpha * acc[i][j][r]);
+        const int m = row0 + 16 * i + g + (r >= 2 ? 8 : 0), n = col0 + 8 * j + 2 * t + (r & 1);
+        const bool v = p.beta != 0.0 && m < p.M && n < p.N && !(p.tri == 1 && m < n) && !(p.tri == 2 && m > n);
+        cc[i][j][r] = v ? p.C[m + (long long)n * p.ldc] : 0.0;
+      }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int m = row0 + 16 * i + g + (r >= 2 ? 8 : 0), n = col0 + 8 * j + 2 * t + (r & 1);
+        const bool v = m < p.M && n < p.N && !(p.tri == 1 && m < n) && !(p.tri == 2 && m > n);
+        const double x = p.beta == 0.0 ? p.alpha * acc[i][j][r] : fma(p.beta, cc[i][j][r], p.alpha * acc[i][j][r]);
+        if (v) p.C[m + (long long)n * p.ldc] = x;
       }
 }
 

@@ -266,7 +266,10 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
   }
 
   // Epilogue: C = alpha * acc + beta * C on the valid (and triangle) region.
-  // All C loads are issued before any store so their latencies overlap.
+  // C is read in groups of eight 16-byte (sixteen 8-byte) loads per thread, all
+  // in flight before the first is used: with a test around each load they ran
+  // one after the other, 27 K cycles per tile against 31 K for the main loop
+  // at K = 128 (two CTAs on the SM).
   const double alpha = p.alpha, beta = p.beta;
   auto row_of = [&](int i, int r) -> int {
     if (AK) return row0 + wm * 64 + i * 16 + g + ((r >= 2) ? 8 : 0);
@@ -286,74 +289,77 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
   // MN-major A: tiles 2pr and 2pr+1 hold rows (2g, 2g+1) -> one 16-byte access
   const bool vec = !AK && p.cvec;
   if (vec) {
+    // a tile wholly inside C (and its triangle) takes no test per element
+    const bool inside = row0 + BM <= p.M && col0 + BN <= p.N && !(p.tri == 1 && row0 < col0 + BN - 1) &&
+                        !(p.tri == 2 && row0 + BM - 1 > col0);
+    double* cbase = p.C + row_of(0, 0);
 #pragma unroll
-    for (int pr = 0; pr < 2; ++pr)
+    for (int h = 0; h < 4; ++h) {  // row pair pr = h / 2, columns tiles j = 2 (h & 1), + 1: eight loads in flight
+      const int pr = h >> 1, j0 = 2 * (h & 1);
+      double2 cc[8];
+      double* cp[8];
+      bool v0[8], v1[8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int e = 0; e < 8; ++e) {
+        const int j = j0 + (e >> 2), r = e & 3;
+        const int row = row_of(2 * pr, r), col = col_of(j, r);
+        cp[e] = cbase + (long long)col * p.ldc + (row - row_of(0, 0));
+        v0[e] = inside || valid(row, col);
+        v1[e] = inside || valid(row + 1, col);
+        cc[e] = make_double2(0.0, 0.0);
+      }
+      if (beta != 0.0) {
+        if (inside) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int row = row_of(2 * pr, r), col = col_of(j, r);
-          const bool v0 = valid(row, col), v1 = valid(row + 1, col);
-          double* cp = p.C + (long long)col * p.ldc + row;
-          double c0 = 0.0, c1 = 0.0;
-          if (beta != 0.0) {
-            if (v0 && v1) {
-              const double2 cc = *reinterpret_cast<const double2*>(cp);
-              c0 = cc.x; c1 = cc.y;
-            } else {
-              if (v0) c0 = cp[0];
-              if (v1) c1 = cp[1];
-            }
-          }
-          acc[2 * pr][j][r] = fma(beta, c0, alpha * acc[2 * pr][j][r]);
-          acc[2 * pr + 1][j][r] = fma(beta, c1, alpha * acc[2 * pr + 1][j][r]);
-        }
+          for (int e = 0; e < 8; ++e) cc[e] = *reinterpret_cast<const double2*>(cp[e]);
+        } else {
 #pragma unroll
-    for (int pr = 0; pr < 2; ++pr)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int row = row_of(2 * pr, r), col = col_of(j, r);
-          const bool v0 = valid(row, col), v1 = valid(row + 1, col);
-          double* cp = p.C + (long long)col * p.ldc + row;
-          if (v0 && v1) {
-            *reinterpret_cast<double2*>(cp) = make_double2(acc[2 * pr][j][r], acc[2 * pr + 1][j][r]);
-          } else {
-            if (v0) cp[0] = acc[2 * pr][j][r];
-            if (v1) cp[1] = acc[2 * pr + 1][j][r];
+          for (int e = 0; e < 8; ++e) {
+            if (v0[e]) cc[e].x = cp[e][0];
+            if (v1[e]) cc[e].y = cp[e][1];
           }
         }
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int j = j0 + (e >> 2), r = e & 3;
+        cc[e].x = fma(beta, cc[e].x, alpha * acc[2 * pr][j][r]);
+        cc[e].y = fma(beta, cc[e].y, alpha * acc[2 * pr + 1][j][r]);
+      }
+      if (inside) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) *reinterpret_cast<double2*>(cp[e]) = cc[e];
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          if (v0[e]) cp[e][0] = cc[e].x;
+          if (v1[e]) cp[e][1] = cc[e].y;
+        }
+      }
+    }
     return;
   }
-  if (beta != 0.0) {
+  const bool inside = row0 + BM <= p.M && col0 + BN <= p.N && !(p.tri == 1 && row0 < col0 + BN - 1) &&
+                      !(p.tri == 2 && row0 + BM - 1 > col0);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int row = row_of(i, r), col = col_of(j, r);
-          const double c = valid(row, col) ? p.C[(long long)col * p.ldc + row] : 0.0;
-          acc[i][j][r] = fma(beta, c, alpha * acc[i][j][r]);
-        }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[i][j][r] *= alpha;
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 4; ++i) {  // sixteen loads in flight
+    double cc[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int row = row_of(i, r), col = col_of(j, r);
-        if (valid(row, col)) p.C[(long long)col * p.ldc + row] = acc[i][j][r];
+        cc[j][r] = beta != 0.0 && (inside || valid(row, col)) ? p.C[(long long)col * p.ldc + row] : 0.0;
       }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row = row_of(i, r), col = col_of(j, r);
+        cc[j][r] = beta != 0.0 ? fma(beta, cc[j][r], alpha * acc[i][j][r]) : alpha * acc[i][j][r];
+        if (inside || valid(row, col)) p.C[(long long)col * p.ldc + row] = cc[j][r];
+      }
+  }
 }
 
 }  // namespace egpu

@@ -33,6 +33,7 @@
 #include <new>
 #include <vector>
 
+#include "diag_common.cuh"
 #include "internal.h"
 
 namespace egpu {
@@ -53,13 +54,15 @@ struct BatchItem {
 constexpr int kBmaxN = 512;                    // largest order handled by one CTA
 constexpr int kBmaxRHS = 16;                   // right-hand sides per system
 constexpr int kRC = 8;                         // right-hand sides per shared-memory chunk
-constexpr int kPLD = kBmaxN + 32;              // panel leading dimension (rows)
+constexpr int kPLD = kBmaxN + 34;              // panel leading dimension (rows; 2 mod 16: conflict-free
+                                               // 16-byte fragment loads at rows 2 g, columns 2 t)
 constexpr int kIRMax = 10;                     // refinement corrections before the FP64 fallback
 constexpr double kIRTol = 1e-14;               // backward error the refined plans reach
 constexpr int kScrDoubles = kBmaxN * 32 + kBmaxN / 2;  // per-CTA scratch: inverses + interchanges
 
 // Shared-memory layout (bytes) for storage type T and panel width NB: the
-// panel P, the diagonal-block inverse / solve staging X (NB x (NB + 1)), the
+// panel P, the diagonal-block inverse / solve staging X (NB x (NB + 4)), the
+// diagonal block in FP64 while it is factored S (the same size), the
 // left-looking dots Y (NB x kRC) and, for refined plans whose panel is
 // smaller than two right-hand-side chunks, the solution chunk BS.  The
 // solves' chunk R (and the refined plans' solution chunk otherwise) alias
@@ -67,14 +70,16 @@ constexpr int kScrDoubles = kBmaxN * 32 + kBmaxN / 2;  // per-CTA scratch: inver
 constexpr size_t kChunkBytes = (size_t)kRC * kBmaxN * 8;
 template <typename T, int NB>
 struct BL {
-  static constexpr int kXLD = NB + 1;
+  static constexpr int kXLD = NB + 4;
   static constexpr size_t kPBytes = (size_t)NB * kPLD * sizeof(T);
   static constexpr bool kOwnBS = sizeof(T) == 4 && kPBytes < 2 * kChunkBytes;
   static constexpr size_t kOffX = (kPBytes + 15) & ~size_t(15);
-  static constexpr size_t kOffY = kOffX + (size_t)NB * kXLD * 8;
+  static constexpr size_t kOffS = kOffX + (size_t)NB * kXLD * 8;
+  static constexpr size_t kOffY = kOffS + (size_t)NB * kXLD * 8;
   static constexpr size_t kOffB = kOffY + (size_t)NB * kRC * 8;
   static constexpr size_t kBytes = kOffB + (kOwnBS ? kChunkBytes : 0);
   static_assert(kPBytes >= kChunkBytes, "the solves' chunk aliases the panel");
+  static_assert((size_t)NB * kXLD * 8 >= 2 * 8 * (2 + NB / 2) * 16, "the panel's candidates (8 warps) fit S");
 };
 
 struct BatchArgs {
@@ -141,21 +146,22 @@ __device__ __forceinline__ void tile_syrk(T* C, long long ldc, bool cvec, const 
                                           int pb) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double acc[2][4][4];
+  // C's loads are all in flight before the first is used (a test around each
+  // would run them one after the other)
+  const bool full = cvec && prow + 32 <= m2 && prow >= pcol + 32;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int row = prow + 2 * g + ((r >= 2) ? 16 : 0);
       const int col = pcol + (j >> 1) * 16 + 2 * (2 * t + (r & 1)) + (j & 1);
-      const bool v0 = row < m2 && col < m2 && row >= col;
-      const bool v1 = row + 1 < m2 && col < m2 && row + 1 >= col;
       const T* cp = C + (long long)col * ldc + row;
       double c0 = 0.0, c1 = 0.0;
-      if (cvec && v0 && v1) {
+      if (full) {
         ld_pair(cp, c0, c1);
       } else {
-        if (v0) c0 = ldv(cp);
-        if (v1) c1 = ldv(cp + 1);
+        if (row < m2 && col < m2 && row >= col) c0 = ldv(cp);
+        if (row + 1 < m2 && col < m2 && row + 1 >= col) c1 = ldv(cp + 1);
       }
       acc[0][j][r] = -c0;
       acc[1][j][r] = -c1;
@@ -194,14 +200,12 @@ __device__ __forceinline__ void tile_syrk(T* C, long long ldc, bool cvec, const 
     for (int r = 0; r < 4; ++r) {
       const int row = prow + 2 * g + ((r >= 2) ? 16 : 0);
       const int col = pcol + (j >> 1) * 16 + 2 * (2 * t + (r & 1)) + (j & 1);
-      const bool v0 = row < m2 && col < m2 && row >= col;
-      const bool v1 = row + 1 < m2 && col < m2 && row + 1 >= col;
       T* cp = C + (long long)col * ldc + row;
-      if (cvec && v0 && v1) {
+      if (full) {
         st_pair(cp, -acc[0][j][r], -acc[1][j][r]);
       } else {
-        if (v0) stv(cp, -acc[0][j][r]);
-        if (v1) stv(cp + 1, -acc[1][j][r]);
+        if (row < m2 && col < m2 && row >= col) stv(cp, -acc[0][j][r]);
+        if (row + 1 < m2 && col < m2 && row + 1 >= col) stv(cp + 1, -acc[1][j][r]);
       }
     }
 }
@@ -214,58 +218,57 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
                                           int prow, int pcol, int mrows, int ncols, int pb) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double acc[2][4][4];
+  // C's loads are all in flight before the first is used (a test around each
+  // would run them one after the other)
+  const bool full = cvec && prow + 32 <= mrows && pcol + 32 <= ncols;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int row = prow + 2 * g + ((r >= 2) ? 16 : 0);
       const int col = pcol + 8 * j + 2 * t + (r & 1);
-      const bool v0 = row < mrows && col < ncols;
-      const bool v1 = row + 1 < mrows && col < ncols;
       const T* cp = C + (long long)col * ldc + row;
       double c0 = 0.0, c1 = 0.0;
-      if (cvec && v0 && v1) {
+      if (full) {
         ld_pair(cp, c0, c1);
       } else {
-        if (v0) c0 = ldv(cp);
-        if (v1) c1 = ldv(cp + 1);
+        if (row < mrows && col < ncols) c0 = ldv(cp);
+        if (row + 1 < mrows && col < ncols) c1 = ldv(cp + 1);
       }
       acc[0][j][r] = -c0;
       acc[1][j][r] = -c1;
     }
+  double bf[NB / 8][4][2];  // U's fragments, in flight with C
 #pragma unroll
-  for (int ks = 0; ks < NB / 8; ++ks) {
-    const int ke = ks * 8 + 2 * t;
-    double af[2][4], bf[4][2];
-    {
-      const int m0 = pb + prow + 2 * g;
-      double x00, y00, x01, y01, x10, y10, x11, y11;
-      ld_pair(P + ke * kPLD + m0, x00, y00);
-      ld_pair(P + (ke + 1) * kPLD + m0, x01, y01);
-      ld_pair(P + ke * kPLD + m0 + 16, x10, y10);
-      ld_pair(P + (ke + 1) * kPLD + m0 + 16, x11, y11);
-      af[0][0] = x00; af[0][1] = x10; af[0][2] = x01; af[0][3] = x11;
-      af[1][0] = y00; af[1][1] = y10; af[1][2] = y01; af[1][3] = y11;
-    }
+  for (int ks = 0; ks < NB / 8; ++ks)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int col = pcol + 8 * j + g;
-      bf[j][0] = 0.0;
-      bf[j][1] = 0.0;
-      if (col < ncols) {
-        const T* up = U + (long long)col * ldu + ke;
-        if (cvec) {
-          ld_pair(up, bf[j][0], bf[j][1]);
-        } else {
-          bf[j][0] = ldv(up);
-          bf[j][1] = ldv(up + 1);
-        }
+      const T* up = U + (long long)col * ldu + ks * 8 + 2 * t;
+      bf[ks][j][0] = bf[ks][j][1] = 0.0;
+      if (full) {
+        ld_pair(up, bf[ks][j][0], bf[ks][j][1]);
+      } else if (col < ncols) {
+        bf[ks][j][0] = ldv(up);
+        bf[ks][j][1] = ldv(up + 1);
       }
     }
 #pragma unroll
+  for (int ks = 0; ks < NB / 8; ++ks) {
+    const int ke = ks * 8 + 2 * t;
+    double af[2][4];
+    const int m0 = pb + prow + 2 * g;
+    double x00, y00, x01, y01, x10, y10, x11, y11;
+    ld_pair(P + ke * kPLD + m0, x00, y00);
+    ld_pair(P + (ke + 1) * kPLD + m0, x01, y01);
+    ld_pair(P + ke * kPLD + m0 + 16, x10, y10);
+    ld_pair(P + (ke + 1) * kPLD + m0 + 16, x11, y11);
+    af[0][0] = x00; af[0][1] = x10; af[0][2] = x01; af[0][3] = x11;
+    af[1][0] = y00; af[1][1] = y10; af[1][2] = y01; af[1][3] = y11;
+#pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dmma_16x8x8(acc[i][j], af[i], bf[j]);
+      for (int j = 0; j < 4; ++j) dmma_16x8x8(acc[i][j], af[i], bf[ks][j]);
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -273,57 +276,56 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
     for (int r = 0; r < 4; ++r) {
       const int row = prow + 2 * g + ((r >= 2) ? 16 : 0);
       const int col = pcol + 8 * j + 2 * t + (r & 1);
-      const bool v0 = row < mrows && col < ncols;
-      const bool v1 = row + 1 < mrows && col < ncols;
       T* cp = C + (long long)col * ldc + row;
-      if (cvec && v0 && v1) {
+      if (full) {
         st_pair(cp, -acc[0][j][r], -acc[1][j][r]);
       } else {
-        if (v0) stv(cp, -acc[0][j][r]);
-        if (v1) stv(cp + 1, -acc[1][j][r]);
+        if (row < mrows && col < ncols) stv(cp, -acc[0][j][r]);
+        if (row + 1 < mrows && col < ncols) stv(cp + 1, -acc[1][j][r]);
       }
     }
 }
 
 // ------------------------------------------------ diagonal-block kernels --
-// Lower Cholesky of the b x b top of the panel (b <= NB <= 32) by one warp,
-// the LVar3Unb steps (Cholesky/LVar3.hpp:19-49: alpha11 := sqrt(alpha11),
-// a21 := a21 / alpha11, A22 -= a21 a21^H) with lane r holding row r in
-// registers; the scaling multiplies by the correctly rounded reciprocal.
-// Stores L (rounded to T) into P and 1 / L(i,i) of the stored values into
-// rd.  Returns 0 or the 1-based column of a non-positive pivot (warp-uniform).
+// Lower Cholesky of the b x b top of the panel (b <= NB, NB 16 or 32) and the
+// inverse of its factor (into X, ld NB + 4, lower part) by one warp: the block
+// in FP64 in S (ld NB + 4, padded with identity), factored and inverted in
+// 16-column leaves with the 16 x 16 products between them on DMMA.  The factor
+// goes back to P rounded to T.  Bound by the leaves' chains: 32 columns took
+// 23 us as one unrolled register loop (its code alone 250 KB), 6 us this way.
+// Returns 0 or the 1-based column of a non-positive pivot (warp-uniform).
 template <typename T, int NB>
-__device__ int diag_chol_warp(T* P, int b, double* rd) {
+__device__ int diag_chol_warp(T* P, int b, double* S, double* X, double* col) {
+  constexpr int LD = NB + 4;
   const int lane = threadIdx.x & 31;
-  double a[NB];
-#pragma unroll
-  for (int k = 0; k < NB; ++k) a[k] = (lane < b && k < b && k <= lane) ? ldv(P + k * kPLD + lane) : 0.0;
-  int fail = 0;
-#pragma unroll
-  for (int j = 0; j < NB; ++j) {
-    if (j < b && fail == 0) {
-      const double d = __shfl_sync(0xffffffffu, a[j], j);
-      if (d <= 0.0) {
-        fail = j + 1;
-      } else {
-        const double s = sqrt(d);
-        const double rs = __drcp_rn(s);
-        if (lane == j) a[j] = s;
-        else if (lane > j) a[j] *= rs;
-#pragma unroll
-        for (int k = j + 1; k < NB; ++k) {
-          const double lkj = __shfl_sync(0xffffffffu, a[j], k);
-          if (lane >= k) a[k] = fma(-a[j], lkj, a[k]);
-        }
-      }
+  if (lane < NB) {
+#pragma unroll 8
+    for (int c = 0; c < NB; ++c)
+      if (c <= lane) S[lane + c * LD] = lane < b ? ldv(P + c * kPLD + lane) : (lane == c ? 1.0 : 0.0);
+  }
+  __syncwarp();
+  int f = warp_chol16(S, LD, 0, X, LD, col);
+  if constexpr (NB == 32) {
+    if (f == 0 && b > 16) {
+      smem_dmma_tile16<false, false, true>(S + 16, LD, X, LD, S + 16, LD, 0, 0, 0, 16, 1.0);  // L21 = A21 inv(L11)^T
+      __syncwarp();
+      smem_syrk_tile16<LD>(S + 16, S + 16 + 16 * LD, 0, 0);
+      __syncwarp();
+      f = warp_chol16(S, LD, 16, X + 16 + 16 * LD, LD, col);
+      f = f ? f + 16 : 0;
+      // X21 = -X22 (L21 X11), the product in S's unused upper block
+      smem_dmma_tile16<false, true>(S + 16, LD, X, LD, S + 16 * LD, LD, 0, 0, 0, 16, 1.0);
+      __syncwarp();
+      smem_dmma_tile16<true, false>(X + 16 + 16 * LD, LD, S + 16 * LD, LD, X + 16, LD, 0, 0, 0, 16, -1.0);
+      __syncwarp();
     }
   }
-  if (fail) return fail;
-#pragma unroll
-  for (int k = 0; k < NB; ++k)
-    if (lane < b && k < b && k <= lane) stv(P + k * kPLD + lane, a[k]);
-  __syncwarp();
-  if (lane < b) rd[lane] = __drcp_rn(ldv(P + lane * kPLD + lane));
+  if (f) return f;
+  if (lane < b) {
+#pragma unroll 8
+    for (int c = 0; c < NB; ++c)
+      if (c <= lane) stv(P + c * kPLD + lane, S[lane + c * LD]);
+  }
   __syncwarp();
   return 0;
 }
@@ -367,97 +369,125 @@ __device__ void tri_inv_warp(const T* P, int b, const double* rd, double* out, i
   }
 }
 
-// LU with partial pivoting of the m x b panel in shared memory (lu::Panel,
-// LU/Panel.hpp:19-89: the entry of largest magnitude, the first in row
-// order on ties; zero pivot -> singular; a21 *= 1/alpha11; A22 -= a21 a12).
-// The chosen row is marked done instead of swapped; every thread keeps the
-// current position of the rows it owns (rows tid + t * NT), so the sequential
-// interchange semantics (position j <-> position p_j) hold and a column
-// costs one CTA barrier.  Afterwards the panel rows are permuted into
-// position order in place; s_mv receives the (from, to) row moves and
-// s_piv[j] the position swapped with j at step j.  Returns 0 or the 1-based
-// column of a zero pivot (CTA-uniform).
-template <typename T, int NB, int NT>
-__device__ int lu_panel_smem(T* P, int m, int b, int* s_piv, int* s_mv, int* s_nmv, double* s_rv, int* s_rp,
-                             int* s_rh) {
-  constexpr int RPT = kBmaxN / NT;
-  constexpr int NW = NT / 32;
+// Columns [t0, t1) of lu_panel_smem (WN: the columns that can still be needed
+// from t0 on, a multiple of 8): rolled, register 0 the current column, the
+// rank-1 update rotating the registers.  Returns 0 or the 1-based column of
+// a zero pivot (CTA-uniform).
+template <typename T, int NB, int NT, int WN>
+__device__ __forceinline__ int lu_panel_cols(T (&v)[kBmaxN / NT][NB], int (&pos)[kBmaxN / NT],
+                                             bool (&done)[kBmaxN / NT], T* P, int t0, int t1, int* s_piv,
+                                             double2* candb) {
+  constexpr int RPT = kBmaxN / NT, NW = NT / 32, kMsg = 2 + NB / 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int pos[RPT];
-  bool done[RPT];
-#pragma unroll
-  for (int t = 0; t < RPT; ++t) {
-    pos[t] = tid + t * NT;
-    done[t] = pos[t] >= m;
-  }
-  for (int j = 0; j < b; ++j) {
-    double best = -1.0;
-    int bpos = INT_MAX, bphys = -1;
+#pragma unroll 1
+  for (int j = t0; j < t1; ++j) {
+    double2* cand = candb + (j & 1) * NW * kMsg;
+    // this thread's candidate (a NaN is never one, as it never compares greater)
+    unsigned long long key = 0ull;
+    int kpos = kNoPos, ks = 0;
+    double pv = 1.0;
 #pragma unroll
     for (int t = 0; t < RPT; ++t) {
-      if (!done[t]) {
-        const double v = fabs(ldv(P + j * kPLD + tid + t * NT));
-        if (v > best || (v == best && pos[t] < bpos)) {
-          best = v;
-          bpos = pos[t];
-          bphys = tid + t * NT;
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int op = __shfl_xor_sync(0xffffffffu, bpos, o);
-      const int oh = __shfl_xor_sync(0xffffffffu, bphys, o);
-      if (ob > best || (ob == best && op < bpos)) {
-        best = ob;
-        bpos = op;
-        bphys = oh;
-      }
-    }
-    const int par = (j & 1) * NW;
-    if (lane == 0) {
-      s_rv[par + warp] = best;
-      s_rp[par + warp] = bpos;
-      s_rh[par + warp] = bphys;
-    }
-    __syncthreads();
-    best = s_rv[par];
-    bpos = s_rp[par];
-    bphys = s_rh[par];
-#pragma unroll
-    for (int w = 1; w < NW; ++w) {
-      const double ob = s_rv[par + w];
-      const int op = s_rp[par + w];
-      if (ob > best || (ob == best && op < bpos)) {
-        best = ob;
-        bpos = op;
-        bphys = s_rh[par + w];
-      }
-    }
-    if (bphys < 0) return j + 1;
-    const double pv = ldv(P + j * kPLD + bphys);
-    if (pv == 0.0) return j + 1;
-    if (tid == 0) s_piv[j] = bpos;
-#pragma unroll
-    for (int t = 0; t < RPT; ++t) {
-      if (pos[t] == j) pos[t] = bpos;
-      if (tid + t * NT == bphys) {
-        done[t] = true;
-        pos[t] = j;
+      const unsigned long long kk = abs_key((double)v[t][0]);
+      const bool in = !done[t] && kk <= 0x7ff0000000000000ull;
+      if (in && (kpos == kNoPos || kk > key || (kk == key && pos[t] < kpos))) {
+        key = kk;
+        kpos = pos[t];
+        ks = t;
+        pv = (double)v[t][0];
       }
     }
     const double rp = __drcp_rn(pv);
+    const int wl = warp_argmax(key, kpos);
+    double2* cw = cand + warp * kMsg;
+    if (wl < 0) {
+      if (lane == 0) cw[0] = make_double2(0.0, __hiloint2double(kNoPos, 0));
+    } else if (lane == wl) {
+      cw[0] = make_double2(__longlong_as_double((long long)key), __hiloint2double(kpos, tid + ks * NT));
+      cw[1] = make_double2(rp, pv);
+#pragma unroll
+      for (int t = 0; t < RPT; ++t)
+        if (t == ks)
+#pragma unroll
+          for (int q = 0; q < WN / 2; ++q)
+            cw[2 + q] = make_double2((double)v[t][2 * q + 1], 2 * q + 2 < WN ? (double)v[t][(2 * q + 2) % NB] : 0.0);
+    }
+    __syncthreads();
+    unsigned long long ck = 0ull;
+    int cpos = kNoPos;
+    if (lane < NW) {
+      const double2 h = cand[lane * kMsg];
+      ck = (unsigned long long)__double_as_longlong(h.x);
+      cpos = __double2hiint(h.y);
+    }
+    const int wc = warp_argmax(ck, cpos);
+    if (wc < 0) return j + 1;
+    const double2* wm = cand + wc * kMsg;
+    const double whd = wm[0].y;
+    const int wpos = __double2hiint(whd), wrow = __double2loint(whd);
+    const double2 wi = wm[1];
+    if (wi.y == 0.0) return j + 1;
+    if (tid == 0) s_piv[j] = wpos;
 #pragma unroll
     for (int t = 0; t < RPT; ++t) {
-      if (!done[t]) {
-        const int r = tid + t * NT;
-        const double l = ldv(P + j * kPLD + r) * rp;
-        stv(P + j * kPLD + r, l);
-        for (int c = j + 1; c < b; ++c)
-          stv(P + c * kPLD + r, fma(-l, ldv(P + c * kPLD + bphys), ldv(P + c * kPLD + r)));
+      if (pos[t] == j) pos[t] = wpos;
+      if (tid + t * NT == wrow) {  // the pivot row is final
+        done[t] = true;
+        pos[t] = j;
+#pragma unroll
+        for (int k = 0; k < WN; ++k)
+          if (j + k < NB) P[(j + k) * kPLD + wrow] = v[t][k];
       }
     }
+#pragma unroll
+    for (int t = 0; t < RPT; ++t) {
+      const double l = (double)v[t][0] * wi.x;
+      if (!done[t]) P[j * kPLD + tid + t * NT] = (T)l;
+#pragma unroll
+      for (int q = 0; q < WN / 2; ++q) {
+        const double2 u = wm[2 + q];
+        v[t][2 * q] = (T)fma(-l, u.x, (double)v[t][2 * q + 1]);
+        if (2 * q + 2 < WN) v[t][2 * q + 1] = (T)fma(-l, u.y, (double)v[t][(2 * q + 2) % NB]);
+      }
+      v[t][WN - 1] = T(0);
+    }
+  }
+  return 0;
+}
+
+// LU with partial pivoting of the m x b panel in shared memory (lu::Panel,
+// LU/Panel.hpp:19-89: the entry of largest magnitude, the first in row
+// order on ties; zero pivot -> singular; a21 *= 1/alpha11; A22 -= a21 a12).
+// Every thread holds its rows (tid + t * NT) in registers; the chosen row is
+// marked done instead of swapped and every thread keeps the current position
+// of the rows it owns, so the sequential interchange semantics (position j <->
+// position p_j) hold and a column costs one CTA barrier; finished entries go
+// back to P.  (Updating the panel in shared memory took 2500 cycles per column
+// of a 32-wide panel.)  Afterwards the panel rows are permuted into position
+// order in place; s_mv receives the (from, to) row moves and s_piv[j] the
+// position swapped with j at step j.  candb: 2 * NT / 32 * (2 + NB / 2)
+// double2 of scratch.  Returns 0 or the 1-based column of a zero pivot
+// (CTA-uniform).
+template <typename T, int NB, int NT>
+__device__ int lu_panel_smem(T* P, int m, int b, int* s_piv, int* s_mv, int* s_nmv, double2* candb) {
+  constexpr int RPT = kBmaxN / NT;
+  const int tid = threadIdx.x;
+  int pos[RPT];
+  {
+    T v[RPT][NB];
+    bool done[RPT];
+#pragma unroll
+    for (int t = 0; t < RPT; ++t) {
+      const int r = tid + t * NT;
+      pos[t] = r;
+      done[t] = r >= m;
+#pragma unroll
+      for (int k = 0; k < NB; ++k) v[t][k] = (!done[t] && k < b) ? P[k * kPLD + r] : T(0);
+    }
+    int f = lu_panel_cols<T, NB, NT, NB>(v, pos, done, P, 0, min(b, NB / 2), s_piv, candb);
+    if (f) return f;
+    f = lu_panel_cols<T, NB, NT, NB / 2>(v, pos, done, P, NB / 2, b, s_piv, candb);
+    if (f) return f;
   }
   // the row moves, then the panel rows into position order
   if (tid == 0) *s_nmv = 0;
@@ -492,9 +522,11 @@ __device__ int lu_panel_smem(T* P, int m, int b, int* s_piv, int* s_mv, int* s_n
 
 // ------------------------------------------------------------ factorizations --
 // Shared-memory work areas of one CTA (pointers into the dynamic block plus
-// the static scalars); X is NB x (NB + 1), Y is NB x kBmaxRHS doubles.
+// the static scalars); X and S are NB x (NB + 4), Y is NB x kRC doubles.
 struct BWork {
   double* X;
+  double* S;
+  double* col;  // 32 doubles, the leaf factorization's column
   double* Y;
   double* BS;
   double* rd;
@@ -502,8 +534,6 @@ struct BWork {
   int* piv;
   int* mv;
   int* nmv;
-  int* ri;
-  int* rh;
   int* flag;
 };
 
@@ -512,7 +542,7 @@ struct BWork {
 // blocks, ld NB).  Returns 0 or the 1-based column of a non-positive pivot.
 template <typename T, int NB, int NT>
 __device__ int chol_factor(T* F, long long ldf, int n, T* P, const BWork& w, double* Xg) {
-  constexpr int kXLD = NB + 1;
+  constexpr int kXLD = NB + 4;
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool cvec = (reinterpret_cast<uintptr_t>(F) % (2 * sizeof(T)) == 0) && (ldf % 2 == 0);
   for (int k0 = 0; k0 < n; k0 += NB) {
@@ -522,9 +552,8 @@ __device__ int chol_factor(T* F, long long ldf, int n, T* P, const BWork& w, dou
     cp_async_wait_all();
     __syncthreads();
     if (warp == 0) {
-      const int f = diag_chol_warp<T, NB>(P, b, w.rd);
+      const int f = diag_chol_warp<T, NB>(P, b, w.S, w.X, w.col);
       if (tid == 0) *w.flag = f;
-      if (f == 0) tri_inv_warp<T, NB, false, false>(P, b, w.rd, w.X, kXLD);
     }
     __syncthreads();
     if (*w.flag) {
@@ -581,7 +610,7 @@ __device__ int chol_factor(T* F, long long ldf, int n, T* P, const BWork& w, dou
 // column of a zero pivot.
 template <typename T, int NB, int NT>
 __device__ int lu_factor(T* F, long long ldf, int n, T* P, const BWork& w, double* Xg, int* piv) {
-  constexpr int kXLD = NB + 1;
+  constexpr int kXLD = NB + 4;
   constexpr int NW = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool cvec = (reinterpret_cast<uintptr_t>(F) % (2 * sizeof(T)) == 0) && (ldf % 2 == 0);
@@ -591,7 +620,7 @@ __device__ int lu_factor(T* F, long long ldf, int n, T* P, const BWork& w, doubl
       for (int r = tid; r < m; r += NT) cp_async_el(&P[c * kPLD + r], &F[(long long)(k0 + c) * ldf + k0 + r]);
     cp_async_wait_all();
     __syncthreads();
-    const int f = lu_panel_smem<T, NB, NT>(P, m, b, w.piv, w.mv, w.nmv, w.red, w.ri, w.rh);
+    const int f = lu_panel_smem<T, NB, NT>(P, m, b, w.piv, w.mv, w.nmv, reinterpret_cast<double2*>(w.S));
     if (f) {
       __syncthreads();
       return k0 + f;
@@ -671,6 +700,51 @@ __device__ int lu_factor(T* F, long long ldf, int n, T* P, const BWork& w, doubl
 }
 
 // ------------------------------------------------------------------ solves --
+// Row i of a kept diagonal-block inverse X (NB x NB, ld NB, global) times the
+// block's right-hand side rq (bi entries, shared): the unit lower part (UNIT:
+// rq[i] + sum_{k < i} X(i, k) rq[k]), the lower part (k <= i), the upper part
+// (upper: k >= i) or, TRANS, the lower part's transpose (sum_{k >= i} X(k, i)
+// rq[k]).  All NB loads of the row are in flight at once (a loop over the row
+// waited for L2 every few entries).
+template <int NB, bool UNIT, bool TRANS>
+__device__ __forceinline__ double block_row(const double* X, int i, int bi, const double* rq, bool upper = false) {
+  auto in = [&](int k) { return k < bi && (UNIT ? k < i : (TRANS || upper) ? k >= i : k <= i); };
+  if (i >= bi) return 0.0;
+  double x[NB];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) x[k] = in(k) ? X[TRANS ? k + i * NB : i + k * NB] : 0.0;
+  double s0 = UNIT ? rq[i] : 0.0, s1 = 0.0;
+#pragma unroll
+  for (int k = 0; k < NB; k += 2) {  // an entry outside the part never meets rq (which may not be finite)
+    if (in(k)) s0 = fma(x[k], rq[k], s0);
+    if (in(k + 1)) s1 = fma(x[k + 1], rq[k + 1], s1);
+  }
+  return s0 + s1;
+}
+
+// R[q][r] -= sum_k F(r, k) stage[k + q NB] over the block's bi columns (F at
+// its first column), rows r0 <= r < r1; all of a row's loads in flight.
+template <typename T, int NB, int NT>
+__device__ __forceinline__ void rows_update(const T* F, long long ldf, int bi, int r0, int r1, int nr,
+                                            const double* stage, double* R) {
+  for (int r = r0 + (int)threadIdx.x; r < r1; r += NT) {
+    T l[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) l[k] = k < bi ? F[(long long)k * ldf + r] : T(0);
+#pragma unroll
+    for (int q = 0; q < kRC; ++q)
+      if (q < nr) {
+        double a0 = R[q * kBmaxN + r], a1 = 0.0;
+#pragma unroll
+        for (int k = 0; k < NB; k += 2) {
+          a0 = fma(-(double)l[k], stage[k + q * NB], a0);
+          a1 = fma(-(double)l[k + 1], stage[k + 1 + q * NB], a1);
+        }
+        R[q * kBmaxN + r] = a0 + a1;
+      }
+  }
+}
+
 // R (shared, R[q * kBmaxN + i], nr <= kRC columns) := op(factor)^-1 R, blocked
 // by NB with the diagonal-block inverses in Xg.
 //   LU = false: L L^T (cholesky::SolveAfter, Cholesky/SolveAfter.hpp:20-75):
@@ -682,7 +756,7 @@ __device__ void solve_smem(const T* F, long long ldf, int n, int nr, const doubl
                            const BWork& w) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = NT / 32;
-  double* stage = w.X;  // bi x nr
+  double* stage = w.X;  // NB x nr
   const int nblk = (n + NB - 1) / NB;
   for (int ib = 0; ib < nblk; ++ib) {
     const int i0 = ib * NB, bi = min(NB, n - i0);
@@ -701,96 +775,68 @@ __device__ void solve_smem(const T* F, long long ldf, int n, int nr, const doubl
       __syncthreads();
     }
     const double* Xi = Xg + (size_t)ib * NB * NB;
-    for (int e = tid; e < bi * nr; e += NT) {
-      const int i = e % bi, q = e / bi;
-      const double* rq = R + q * kBmaxN + i0;
-      double s = LU ? rq[i] : 0.0;
-      const int kend = LU ? i : i + 1;
-      for (int k = 0; k < kend; ++k) s = fma(Xi[i + k * NB], rq[k], s);
-      stage[e] = s;
+    for (int e = tid; e < NB * nr; e += NT) {
+      const int i = e % NB, q = e / NB;
+      stage[e] = block_row<NB, LU, false>(Xi, i, bi, R + q * kBmaxN + i0);
     }
     __syncthreads();
-    for (int e = tid; e < bi * nr; e += NT) R[(e / bi) * kBmaxN + i0 + e % bi] = stage[e];
-    for (int r = i0 + bi + tid; r < n; r += NT) {
-      double acc[kRC];
-#pragma unroll
-      for (int q = 0; q < kRC; ++q) acc[q] = 0.0;
-      for (int k = 0; k < bi; ++k) {
-        const double l = ldv(F + (long long)(i0 + k) * ldf + r);
-#pragma unroll
-        for (int q = 0; q < kRC; ++q)
-          if (q < nr) acc[q] = fma(l, stage[k + q * bi], acc[q]);
-      }
-#pragma unroll
-      for (int q = 0; q < kRC; ++q)
-        if (q < nr) R[q * kBmaxN + r] -= acc[q];
-    }
+    for (int e = tid; e < NB * nr; e += NT)
+      if (e % NB < bi) R[(e / NB) * kBmaxN + i0 + e % NB] = stage[e];
+    rows_update<T, NB, NT>(F + (long long)i0 * ldf, ldf, bi, i0 + bi, n, nr, stage, R);
     __syncthreads();
   }
   for (int ib = nblk - 1; ib >= 0; --ib) {
     const int i0 = ib * NB, bi = min(NB, n - i0);
     const double* Xi = Xg + (size_t)ib * NB * NB;
     if (!LU) {
-      // D = L(below, block)^T X(below): one warp per column, lanes over rows
-      double* D = w.Y;  // bi x nr
-      for (int c = warp; c < bi; c += NW) {
-        double acc[kRC];
+      // D = L(below, block)^T X(below): a warp takes NB / NW columns at once,
+      // lanes over rows (their loads in flight together, X read once for all)
+      constexpr int CPW = (NB + NW - 1) / NW;
+      double* D = w.Y;  // NB x nr
+      double acc[CPW][kRC];
 #pragma unroll
-        for (int q = 0; q < kRC; ++q) acc[q] = 0.0;
-        const T* lc = F + (long long)(i0 + c) * ldf;
-        for (int r = i0 + bi + lane; r < n; r += 32) {
-          const double l = ldv(lc + r);
+      for (int u = 0; u < CPW; ++u)
 #pragma unroll
-          for (int q = 0; q < kRC; ++q)
-            if (q < nr) acc[q] = fma(l, R[q * kBmaxN + r], acc[q]);
-        }
+        for (int q = 0; q < kRC; ++q) acc[u][q] = 0.0;
+      const T* lc = F + (long long)(i0 + warp * CPW) * ldf;
+#pragma unroll 2
+      for (int r = i0 + bi + lane; r < n; r += 32) {
+        double l[CPW];
 #pragma unroll
-        for (int q = 0; q < kRC; ++q) {
-          if (q < nr) {
-            double v = acc[q];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) D[c + q * bi] = v;
-          }
-        }
-      }
-      __syncthreads();
-      for (int e = tid; e < bi * nr; e += NT) {
-        const int i = e % bi, q = e / bi;
-        const double* rq = R + q * kBmaxN + i0;
-        double s = 0.0;
-        for (int k = i; k < bi; ++k) s = fma(Xi[k + i * NB], rq[k] - D[k + q * bi], s);
-        stage[e] = s;
-      }
-      __syncthreads();
-      for (int e = tid; e < bi * nr; e += NT) R[(e / bi) * kBmaxN + i0 + e % bi] = stage[e];
-      __syncthreads();
-    } else {
-      for (int e = tid; e < bi * nr; e += NT) {
-        const int i = e % bi, q = e / bi;
-        const double* rq = R + q * kBmaxN + i0;
-        double s = 0.0;
-        for (int k = i; k < bi; ++k) s = fma(Xi[i + k * NB], rq[k], s);
-        stage[e] = s;
-      }
-      __syncthreads();
-      for (int e = tid; e < bi * nr; e += NT) R[(e / bi) * kBmaxN + i0 + e % bi] = stage[e];
-      for (int r = tid; r < i0; r += NT) {
-        double acc[kRC];
-#pragma unroll
-        for (int q = 0; q < kRC; ++q) acc[q] = 0.0;
-        for (int k = 0; k < bi; ++k) {
-          const double u = ldv(F + (long long)(i0 + k) * ldf + r);
-#pragma unroll
-          for (int q = 0; q < kRC; ++q)
-            if (q < nr) acc[q] = fma(u, stage[k + q * bi], acc[q]);
-        }
+        for (int u = 0; u < CPW; ++u) l[u] = warp * CPW + u < bi ? ldv(lc + (long long)u * ldf + r) : 0.0;
 #pragma unroll
         for (int q = 0; q < kRC; ++q)
-          if (q < nr) R[q * kBmaxN + r] -= acc[q];
+          if (q < nr) {
+            const double x = R[q * kBmaxN + r];
+#pragma unroll
+            for (int u = 0; u < CPW; ++u) acc[u][q] = fma(l[u], x, acc[u][q]);
+          }
       }
+#pragma unroll
+      for (int q = 0; q < kRC; ++q)
+        if (q < nr) {
+#pragma unroll
+          for (int u = 0; u < CPW; ++u) {
+            double v = acc[u][q];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0 && warp * CPW + u < NB) D[warp * CPW + u + q * NB] = v;
+          }
+        }
+      __syncthreads();
+      for (int e = tid; e < NB * nr; e += NT)
+        if (e % NB < bi) R[(e / NB) * kBmaxN + i0 + e % NB] -= D[e];
       __syncthreads();
     }
+    for (int e = tid; e < NB * nr; e += NT) {
+      const int i = e % NB, q = e / NB;
+      stage[e] = block_row<NB, false, !LU>(Xi, i, bi, R + q * kBmaxN + i0, LU);
+    }
+    __syncthreads();
+    for (int e = tid; e < NB * nr; e += NT)
+      if (e % NB < bi) R[(e / NB) * kBmaxN + i0 + e % NB] = stage[e];
+    if (LU) rows_update<T, NB, NT>(F + (long long)i0 * ldf, ldf, bi, 0, i0, nr, stage, R);
+    __syncthreads();
   }
 }
 
@@ -946,14 +992,16 @@ __global__ void __launch_bounds__(NT, MINB) batched_kernel(BatchArgs args) {
   constexpr bool kRefined = sizeof(T) == 4;
   constexpr bool kHPD = KIND == 0;
   __shared__ double s_rd[32];
+  __shared__ __align__(16) double s_col[32];
   __shared__ double s_red[3 * kRC * (NT / 32) + 3 * kRC];
   __shared__ int s_piv[32];
   __shared__ int s_mv[2 * 64];
   __shared__ int s_nmv, s_idx, s_flag;
-  __shared__ int s_ri[2 * (NT / 32)], s_rh[2 * (NT / 32)];
   T* P = reinterpret_cast<T*>(sm_dyn);
   BWork w;
   w.X = reinterpret_cast<double*>(sm_dyn + LY::kOffX);
+  w.S = reinterpret_cast<double*>(sm_dyn + LY::kOffS);
+  w.col = s_col;
   w.Y = reinterpret_cast<double*>(sm_dyn + LY::kOffY);
   w.BS = reinterpret_cast<double*>(sm_dyn + (LY::kOwnBS ? LY::kOffB : kChunkBytes));
   w.rd = s_rd;
@@ -961,8 +1009,6 @@ __global__ void __launch_bounds__(NT, MINB) batched_kernel(BatchArgs args) {
   w.piv = s_piv;
   w.mv = s_mv;
   w.nmv = &s_nmv;
-  w.ri = s_ri;
-  w.rh = s_rh;
   w.flag = &s_flag;
   const int tid = threadIdx.x;
   double* Xg = args.scratch + (size_t)blockIdx.x * kScrDoubles;

@@ -25,6 +25,33 @@ constexpr int kDiagSmemBase = (128 * kLDS + 128) * (int)sizeof(double);
 template <typename T>
 __device__ __forceinline__ T& SE(T* S, int r, int c) { return S[r + c * kLDS]; }
 
+// ------------------------------------------------------------ pivot search --
+constexpr int kNoPos = 0x7fffffff;  // "no row": a lane that does not take part
+
+// |a| as a key whose unsigned order is the order of |a| (non-negative doubles)
+__device__ __forceinline__ unsigned long long abs_key(double v) {
+  return (unsigned long long)__double_as_longlong(fabs(v));
+}
+
+// The rare part of warp_argmax, out of line (the column loops are short of
+// instruction-cache room): the upper halves tie.
+static __device__ __noinline__ unsigned warp_argmax_tie(bool c, unsigned lo, int pos) {
+  const unsigned ml = __reduce_max_sync(0xffffffffu, c ? lo : 0u);
+  const unsigned r = __reduce_min_sync(0xffffffffu, c && lo == ml ? (unsigned)pos : (unsigned)kNoPos);
+  return __ballot_sync(0xffffffffu, c && lo == ml && (unsigned)pos == r);
+}
+
+// Lane of the first maximal key over the lanes with pos != kNoPos, ties to
+// the lowest position; -1 when no lane takes part.
+__device__ __forceinline__ int warp_argmax(unsigned long long key, int pos) {
+  const bool in = pos != kNoPos;
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, in ? hi : 0u);
+  unsigned m = __ballot_sync(0xffffffffu, in && hi == mh);
+  if (__popc(m) > 1) m = warp_argmax_tie(in && hi == mh, lo, pos);  // warp-uniform
+  return __ffs(m) - 1;
+}
+
 // ---------------------------------------------------------------------------
 // Building blocks on shared-memory operands (all column-major).
 
@@ -184,11 +211,14 @@ __device__ inline int pad16_identity(double* S, int b) {
 }
 
 // One 16 x 16 tile (two 16 x 8 DMMA columns) of a product of shared-memory
-// operands, k in [kbeg, kend): C = alpha A B.  A_LOWER / B_LOWER: A (B) is
-// zero above its diagonal and what is stored there is not used.
-template <bool A_LOWER, bool B_LOWER>
+// operands by one warp, k in [kbeg, kend): C = alpha A op(B).  A_LOWER /
+// B_LOWER: A (B) is zero above its diagonal and what is stored there is not
+// used.  B_TRANS: op(B) = B^T.  C may be A (this tile's rows and k columns):
+// every lane has read before any writes.
+template <bool A_LOWER, bool B_LOWER, bool B_TRANS = false>
 __device__ __forceinline__ void smem_dmma_tile16(const double* A, int lda, const double* B, int ldb, double* C,
                                                  int ldc, int r0, int c0, int kbeg, int kend, double alpha) {
+  static_assert(!(B_LOWER && B_TRANS), "not needed");
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double acc0[4] = {0.0, 0.0, 0.0, 0.0}, acc1[4] = {0.0, 0.0, 0.0, 0.0};
   const int ra = r0 + g, rb = r0 + g + 8, ca = c0 + g, cb = c0 + g + 8;
@@ -200,13 +230,14 @@ __device__ __forceinline__ void smem_dmma_tile16(const double* A, int lda, const
     a[1] = (!A_LOWER || ka <= rb) ? A[rb + ka * lda] : 0.0;
     a[2] = (!A_LOWER || kb <= ra) ? A[ra + kb * lda] : 0.0;
     a[3] = (!A_LOWER || kb <= rb) ? A[rb + kb * lda] : 0.0;
-    b0[0] = (!B_LOWER || ca <= ka) ? B[ka + ca * ldb] : 0.0;
-    b0[1] = (!B_LOWER || ca <= kb) ? B[kb + ca * ldb] : 0.0;
-    b1[0] = (!B_LOWER || cb <= ka) ? B[ka + cb * ldb] : 0.0;
-    b1[1] = (!B_LOWER || cb <= kb) ? B[kb + cb * ldb] : 0.0;
+    b0[0] = (!B_LOWER || ca <= ka) ? (B_TRANS ? B[ca + ka * ldb] : B[ka + ca * ldb]) : 0.0;
+    b0[1] = (!B_LOWER || ca <= kb) ? (B_TRANS ? B[ca + kb * ldb] : B[kb + ca * ldb]) : 0.0;
+    b1[0] = (!B_LOWER || cb <= ka) ? (B_TRANS ? B[cb + ka * ldb] : B[ka + cb * ldb]) : 0.0;
+    b1[1] = (!B_LOWER || cb <= kb) ? (B_TRANS ? B[cb + kb * ldb] : B[kb + cb * ldb]) : 0.0;
     dmma_16x8x8(acc0, a, b0);
     dmma_16x8x8(acc1, a, b1);
   }
+  __syncwarp();
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int r = r0 + g + ((q >= 2) ? 8 : 0), c = c0 + 2 * t + (q & 1);
@@ -255,8 +286,9 @@ __device__ inline void smem_trinv_dmma(double* S, int bp, const double* Xl, doub
   }
 }
 
-// C(r0.., c0..) -= A(r0.., 0..15) A(c0.., 0..15)^T on one 16 x 16 tile (all ld
-// kLDS); on the diagonal (r0 == c0) only the lower triangle is written.
+// C(r0.., c0..) -= A(r0.., 0..15) A(c0.., 0..15)^T on one 16 x 16 tile (both ld
+// LD); on the diagonal (r0 == c0) only the lower triangle is written.
+template <int LD = kLDS>
 __device__ __forceinline__ void smem_syrk_tile16(const double* A, double* C, int r0, int c0) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double acc[2][4];
@@ -264,19 +296,19 @@ __device__ __forceinline__ void smem_syrk_tile16(const double* A, double* C, int
   for (int h = 0; h < 2; ++h)
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      acc[h][q] = C[(r0 + g + ((q >= 2) ? 8 : 0)) + (c0 + 8 * h + 2 * t + (q & 1)) * kLDS];
+      acc[h][q] = C[(r0 + g + ((q >= 2) ? 8 : 0)) + (c0 + 8 * h + 2 * t + (q & 1)) * LD];
   double a[2][4], b[2][2][2];
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    const double* ak = A + (8 * u + t) * kLDS + g;
+    const double* ak = A + (8 * u + t) * LD + g;
     a[u][0] = -ak[r0];
     a[u][1] = -ak[r0 + 8];
-    a[u][2] = -ak[r0 + 4 * kLDS];
-    a[u][3] = -ak[r0 + 8 + 4 * kLDS];
+    a[u][2] = -ak[r0 + 4 * LD];
+    a[u][3] = -ak[r0 + 8 + 4 * LD];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       b[u][h][0] = ak[c0 + 8 * h];
-      b[u][h][1] = ak[c0 + 8 * h + 4 * kLDS];
+      b[u][h][1] = ak[c0 + 8 * h + 4 * LD];
     }
   }
 #pragma unroll
@@ -288,7 +320,7 @@ __device__ __forceinline__ void smem_syrk_tile16(const double* A, double* C, int
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int r = r0 + g + ((q >= 2) ? 8 : 0), c = c0 + 8 * h + 2 * t + (q & 1);
-      if (r0 != c0 || r >= c) C[r + c * kLDS] = acc[h][q];
+      if (r0 != c0 || r >= c) C[r + c * LD] = acc[h][q];
     }
 }
 

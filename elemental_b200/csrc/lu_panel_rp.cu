@@ -72,7 +72,6 @@ constexpr int kRpWarps = kRpThreads / 32;  // also the most column warps
 constexpr int kRpW = 16;         // sub-panel width
 constexpr int kRpMsg = 10;       // double2 per candidate: {|a|, position : row}, {1 / pivot, pivot}, u[0..14]
 constexpr int kRpMaxCl = 16;
-constexpr int kRpNoPos = 0x7fffffff;
 constexpr int kRpLdU = 132;      // 4 mod 16: conflict-free DMMA fragment loads
 
 // shared-memory layout (in doubles); the sub-panel copy Lb is [16][R + 4] at the end
@@ -87,27 +86,6 @@ constexpr uint32_t kRpColBytes(int P) { return (uint32_t)(P * kRpMsg * 16); }
 constexpr int rp_smem_doubles(int R) {
   const int work = kRpOffLb + kRpW * (R + 4) + 32;  // + the last tile's rows past R (read, not stored)
   return work > kRpInvDoubles ? work : kRpInvDoubles;
-}
-
-// |a| as a key whose unsigned order is the order of |a| (non-negative doubles)
-__device__ __forceinline__ unsigned long long abs_key(double v) {
-  return (unsigned long long)__double_as_longlong(fabs(v));
-}
-
-// Lane of the first maximal key over the lanes with pos != kRpNoPos, ties to
-// the lowest position; -1 when no lane takes part.
-__device__ __forceinline__ int warp_argmax(unsigned long long key, int pos) {
-  const bool in = pos != kRpNoPos;
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned mh = __reduce_max_sync(0xffffffffu, in ? hi : 0u);
-  unsigned m = __ballot_sync(0xffffffffu, in && hi == mh);
-  if (__popc(m) > 1) {  // warp-uniform
-    const bool c = in && hi == mh;
-    const unsigned ml = __reduce_max_sync(0xffffffffu, c ? lo : 0u);
-    const unsigned r = __reduce_min_sync(0xffffffffu, c && lo == ml ? (unsigned)pos : (unsigned)kRpNoPos);
-    m = __ballot_sync(0xffffffffu, c && lo == ml && (unsigned)pos == r);
-  }
-  return __ffs(m) - 1;
 }
 
 // 32-bit shared::cluster address of the same object in CTA `rank`
@@ -211,13 +189,13 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
     if (!stop && tid < CT) {
       // ---- load the sub-panel rows into registers (own rows >= c0; .cg: no stale L1)
       double v[RT][kRpW];
-      int pos[RT];      // the row's position; kRpNoPos: not a row of the sub-panel
+      int pos[RT];      // the row's position; kNoPos: not a row of the sub-panel
       bool done[RT];    // already a pivot row
 #pragma unroll
       for (int s = 0; s < RT; ++s) {
         const int lr = s * CT + tid;
         const bool act = lr < rows && r0 + lr >= c0;
-        pos[s] = act ? r0 + lr : kRpNoPos;
+        pos[s] = act ? r0 + lr : kNoPos;
         done[s] = !act;
       }
       {
@@ -238,12 +216,12 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
         double2* CAND = CANDB + par * kRpWarps * kRpMsg;
         // 1. the warp's candidate; its owner stages it
         unsigned long long key = 0ull;
-        int kpos = kRpNoPos, ks = 0;
+        int kpos = kNoPos, ks = 0;
         double pv0 = 1.0;
 #pragma unroll
         for (int s = 0; s < RT; ++s) {  // branch-free: a row that is done counts as |a| = 0 at no position
           const unsigned long long kk = done[s] ? 0ull : abs_key(v[s][0]);
-          const int kp = done[s] ? kRpNoPos : pos[s];
+          const int kp = done[s] ? kNoPos : pos[s];
           const bool better = kk > key || (kk == key && kp < kpos);
           key = better ? kk : key;
           kpos = better ? kp : kpos;
@@ -254,7 +232,7 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
         const int wl = warp_argmax(key, kpos);
         double2* cw = &CAND[warp * kRpMsg];
         if (wl < 0) {
-          if (lane == 0) cw[0] = make_double2(0.0, __hiloint2double(kRpNoPos, 0));
+          if (lane == 0) cw[0] = make_double2(0.0, __hiloint2double(kNoPos, 0));
         } else if (lane == wl) {
           cw[0] = make_double2(__longlong_as_double((long long)key),
                                __hiloint2double(kpos, r0 + ks * CT + tid));
@@ -277,7 +255,7 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
         if (P > 1) {
           {
             unsigned long long ck = 0ull;
-            int cpos = kRpNoPos;
+            int cpos = kNoPos;
             if (lane < CW) {
               const double2 h = CAND[lane * kRpMsg];
               ck = (unsigned long long)__double_as_longlong(h.x);
@@ -324,7 +302,7 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
         // the winner (first maximal |a|, lowest position on ties)
         {
           unsigned long long gk = 0ull;
-          int gp = kRpNoPos;
+          int gp = kNoPos;
           if (lane < (P > 1 ? P : CW)) {
             const double2 h = cand[lane * kRpMsg];
             gk = (unsigned long long)__double_as_longlong(h.x);
@@ -363,7 +341,7 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
         for (int s = 0; s < RT; ++s) {
           const int lr = s * CT + tid;
           if (pos[s] == j) pos[s] = wpos;
-          if (r0 + lr == wrow && pos[s] != kRpNoPos) {
+          if (r0 + lr == wrow && pos[s] != kNoPos) {
             pos[s] = j;
             done[s] = true;
 #pragma unroll
@@ -387,7 +365,7 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
         // ---- write the sub-panel back, every row to its new position
 #pragma unroll
         for (int s = 0; s < RT; ++s) {
-          if (pos[s] != kRpNoPos) {
+          if (pos[s] != kNoPos) {
             double* dst = A + (long long)c0 * lda + pos[s];
             const double* from = Lb + s * CT + tid;
 #pragma unroll 4

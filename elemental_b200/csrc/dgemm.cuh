@@ -187,8 +187,11 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
       if (AK) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int r0 = wm * 64 + i * 16 + g;
-          const int r1 = r0 + 8;
+          // the same row interleaving as for MN-major A (a thread's rows 2g, 2g + 1
+          // are adjacent, for the 16-byte epilogue); its even rows meet two to a
+          // bank, which the DMMA pipe hides
+          const int r0 = wm * 64 + (i >> 1) * 32 + 2 * g + (i & 1);
+          const int r1 = r0 + 16;
           const int ch = ks * 4 + t;
           const double2 v0 = *reinterpret_cast<const double2*>(sA + r0 * 16 + ((ch ^ (r0 & 7)) << 1));
           const double2 v1 = *reinterpret_cast<const double2*>(sA + r1 * 16 + ((ch ^ (r1 & 7)) << 1));
@@ -272,7 +275,6 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
   // at K = 128 (two CTAs on the SM).
   const double alpha = p.alpha, beta = p.beta;
   auto row_of = [&](int i, int r) -> int {
-    if (AK) return row0 + wm * 64 + i * 16 + g + ((r >= 2) ? 8 : 0);
     return row0 + wm * 64 + (i >> 1) * 32 + 2 * g + (i & 1) + ((r >= 2) ? 16 : 0);
   };
   auto col_of = [&](int j, int r) -> int {
@@ -286,8 +288,8 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
     if (p.tri == 2 && row > col) return false;
     return true;
   };
-  // MN-major A: tiles 2pr and 2pr+1 hold rows (2g, 2g+1) -> one 16-byte access
-  const bool vec = !AK && p.cvec;
+  // tiles 2pr and 2pr+1 hold rows (2g, 2g+1) -> one 16-byte access
+  const bool vec = p.cvec;
   if (vec) {
     // a tile wholly inside C (and its triangle) takes no test per element
     const bool inside = row0 + BM <= p.M && col0 + BN <= p.N && !(p.tri == 1 && row0 < col0 + BN - 1) &&

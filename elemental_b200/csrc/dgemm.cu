@@ -54,26 +54,15 @@ bool make_tma_2d(CUtensorMap* m, int dtype, const void* base, uint64_t inner, ui
   return r == CUDA_SUCCESS;
 }
 
-static int sm_count_of_current_device() {
-  static int cache[32] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 32 && cache[dev] > 0) return cache[dev];
-  int n = 0;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  if (dev >= 0 && dev < 32) cache[dev] = n;
-  return n;
-}
-
 bool tma_compatible(const void* p, long long ld) {
   return (reinterpret_cast<uintptr_t>(p) % 16 == 0) && (ld % 2 == 0) && ld > 0;
 }
 
-template <bool AK, bool BK, int WM, int WN>
+template <bool AK, bool BK, int WM, int WN, int MI>
 static cudaError_t launch_variant(cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb,
                                   const GemmParams& p, long long nblocks) {
-  using S = GemmShape<WM, WN>;
-  auto kern = dgemm_tma_kernel<AK, BK, WM, WN>;
+  using S = GemmShape<WM, WN, MI>;
+  auto kern = dgemm_tma_kernel<AK, BK, WM, WN, MI>;
   static unsigned attr_mask = 0;  // per template instance, one bit per device
   int dev = 0;
   cudaGetDevice(&dev);
@@ -281,24 +270,21 @@ static int launch_dgemm_small(cudaStream_t st, bool a_kmajor, bool b_kmajor, int
 //   a_kmajor = true : A stored K x M column-major (op = TRANSPOSE)
 //   b_kmajor = true : B stored K x N column-major (op = NORMAL)
 //   b_kmajor = false: B stored N x K column-major (op = TRANSPOSE)
-// wide = true selects a 128-column tile, which keeps whole 128-wide row panels
-// inside one CTA (in-place multiply by an inverted triangle): 128 x 128 (8
-// warps), or 64 x 128 (4 warps, 2 CTAs/SM) when A is MN-major and 128-row
-// tiles would not fill the SMs twice over.
+// wide = true (MN-major A) selects a 64 x 128 tile, which keeps whole 128-wide
+// row panels inside one CTA (in-place multiply by an inverted triangle).
 int launch_dgemm(cudaStream_t st, bool a_kmajor, bool b_kmajor, int M, int N, int K, double alpha,
                  const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
                  long long ldc, int tri, bool wide, DevStatus* status) {
   if (M <= 0 || N <= 0) return EGPU_OK;
   if (K <= 0) return launch_scale(st, M, N, beta, C, ldc, tri);
   if (!tma_compatible(A, lda) || !tma_compatible(B, ldb)) return EGPU_ERR_ALIGN;
-  if (tri != 0 && wide) return EGPU_ERR_ARG;
+  if (wide && (tri != 0 || a_kmajor)) return EGPU_ERR_ARG;
   {
     const int rc = launch_dgemm_small(st, a_kmajor, b_kmajor, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tri,
                                       status);
     if (rc != EGPU_ERR_UNSUPPORTED) return rc;
   }
-  const bool half = wide && !a_kmajor && (M + 127) / 128 < 2 * sm_count_of_current_device();
-  const int BM = half ? 64 : 128, BN = wide ? 128 : 64;
+  const int BM = wide ? 64 : 128, BN = wide ? 128 : 64;
   CUtensorMap ma, mb;
   // K-major: one {16 k, BM} box per stage; MN-major: BM / 16 boxes of
   // {16 m, 16 k} (both 128B-swizzled, see dgemm.cuh)
@@ -322,6 +308,7 @@ int launch_dgemm(cudaStream_t st, bool a_kmajor, bool b_kmajor, int M, int N, in
       nblocks += std::max(0, hi - lo);
     }
   }
+  if (nblocks > 0x3fffffff) return EGPU_ERR_UNSUPPORTED;
   // entries of C the product touches: the whole M x N block, or the lower
   // (tri 1) / upper (tri 2) trapezoid -- a launch over rows [c0, n) of block
   // columns [c0, c1) is a triangle on top of a rectangle
@@ -331,19 +318,23 @@ int launch_dgemm(cudaStream_t st, bool a_kmajor, bool b_kmajor, int M, int N, in
   const double bytes = 8.0 * ((double)M * K + (double)N * K + (beta == 0.0 ? 1.0 : 2.0) * entries);
   TraceMark tm(st, beta == 0.0 ? kTraceTrsm : kTraceUpdate, flops, bytes);
   cudaError_t e;
-  if (half) {
-    if (!b_kmajor) e = launch_variant<false, false, 1, 4>(st, ma, mb, p, nblocks);
-    else e = launch_variant<false, true, 1, 4>(st, ma, mb, p, nblocks);
-  } else if (wide) {
-    if (!a_kmajor && !b_kmajor) e = launch_variant<false, false, 2, 4>(st, ma, mb, p, nblocks);
-    else if (!a_kmajor && b_kmajor) e = launch_variant<false, true, 2, 4>(st, ma, mb, p, nblocks);
-    else if (a_kmajor && !b_kmajor) e = launch_variant<true, false, 2, 4>(st, ma, mb, p, nblocks);
-    else e = launch_variant<true, true, 2, 4>(st, ma, mb, p, nblocks);
+  // warps of 64 x 32 for long k loops that fill the chip several times (the
+  // deferred Herk of the grouped Cholesky), of 32 x 32 for the rest: n = 8192,
+  // C full NT, K = 128 0.73 and 0.65 ms, 512 2.31 and 2.30, 2048 8.47 and 8.70
+  const bool big = K >= 1024 && nblocks >= 1184;  // four CTAs a slot on 148 SMs
+  if (wide) {
+    if (!b_kmajor) e = launch_variant<false, false, 2, 4, 2>(st, ma, mb, p, nblocks);
+    else e = launch_variant<false, true, 2, 4, 2>(st, ma, mb, p, nblocks);
+  } else if (big) {
+    if (!a_kmajor && !b_kmajor) e = launch_variant<false, false, 2, 2, 4>(st, ma, mb, p, nblocks);
+    else if (!a_kmajor && b_kmajor) e = launch_variant<false, true, 2, 2, 4>(st, ma, mb, p, nblocks);
+    else if (a_kmajor && !b_kmajor) e = launch_variant<true, false, 2, 2, 4>(st, ma, mb, p, nblocks);
+    else e = launch_variant<true, true, 2, 2, 4>(st, ma, mb, p, nblocks);
   } else {
-    if (!a_kmajor && !b_kmajor) e = launch_variant<false, false, 2, 2>(st, ma, mb, p, nblocks);
-    else if (!a_kmajor && b_kmajor) e = launch_variant<false, true, 2, 2>(st, ma, mb, p, nblocks);
-    else if (a_kmajor && !b_kmajor) e = launch_variant<true, false, 2, 2>(st, ma, mb, p, nblocks);
-    else e = launch_variant<true, true, 2, 2>(st, ma, mb, p, nblocks);
+    if (!a_kmajor && !b_kmajor) e = launch_variant<false, false, 4, 2, 2>(st, ma, mb, p, nblocks);
+    else if (!a_kmajor && b_kmajor) e = launch_variant<false, true, 4, 2, 2>(st, ma, mb, p, nblocks);
+    else if (a_kmajor && !b_kmajor) e = launch_variant<true, false, 4, 2, 2>(st, ma, mb, p, nblocks);
+    else e = launch_variant<true, true, 4, 2, 2>(st, ma, mb, p, nblocks);
   }
   if (e != cudaSuccess) {
     set_last_error(e, "dgemm launch", __FILE__, __LINE__);

@@ -45,9 +45,20 @@ struct GemmParams {
 constexpr int kBK = 16;
 constexpr int kStages = 4;
 
-template <int WARPS_M, int WARPS_N>
+// Warps of (16 MI) x 32, two CTAs per SM, one tile per CTA.  MI = 2: eight
+// warps, so that a CTA alone on its SM (a small product, or the other CTA in
+// its epilogue) still fills the DMMA pipe; MI = 4: four warps with fewer
+// fragment loads per DMMA, the better one for long k loops on a full chip
+// (launch_dgemm chooses).  n = 16384, K = 128 (C full, NT): 2.81 ms with MI = 4,
+// 2.49 with MI = 2 (0.74 of the DMMA rate); n = 8192, K = 2048 (NN): 8.09 and
+// 8.46 ms (0.91, 0.87).  Several tiles per CTA with the next tile's loads under
+// the epilogue measured slower (0.67 with four, 0.66 with eight at K = 128): the
+// two CTAs of an SM then stay in step, both in the main loop and both in the
+// epilogue, where one tile per CTA lets them drift apart; two groups of four
+// warps taking turns in one CTA 0.51.
+template <int WARPS_M, int WARPS_N, int MI>
 struct GemmShape {
-  static constexpr int BM = 64 * WARPS_M;
+  static constexpr int BM = 16 * MI * WARPS_M;
   static constexpr int BN = 32 * WARPS_N;
   static constexpr int kThreads = 32 * WARPS_M * WARPS_N;
   static constexpr int kStageBytes = (BM + BN) * kBK * 8;
@@ -74,10 +85,10 @@ __device__ __forceinline__ long long tri_cum_upper(int j, int MT) {
 }
 
 __device__ __forceinline__ bool map_tile(const GemmParams& p, int& ti, int& tj) {
-  const long long L = blockIdx.x;
+  const int L = (int)blockIdx.x;
   if (p.tri == 0) {
-    ti = (int)(L % p.tiles_m);
-    tj = (int)(L / p.tiles_m);
+    ti = L % p.tiles_m;
+    tj = L / p.tiles_m;
     return tj < p.tiles_n;
   }
   int lo = 0, hi = p.tiles_n;  // find largest j with cum(j) <= L
@@ -95,21 +106,18 @@ __device__ __forceinline__ bool map_tile(const GemmParams& p, int& ti, int& tj) 
   return ti < p.tiles_m && tj < p.tiles_n;
 }
 
-template <bool AK, bool BK, int WARPS_M, int WARPS_N>
-__global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 4) ? 2 : 1)
+template <bool AK, bool BK, int WARPS_M, int WARPS_N, int MI>
+__global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, 2)
     dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const GemmParams p) {
-  using S = GemmShape<WARPS_M, WARPS_N>;
+  using S = GemmShape<WARPS_M, WARPS_N, MI>;
   constexpr int BM = S::BM, BN = S::BN;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * S::kStageBytes);
   uint64_t* empty = full + kStages;  // one arrival per warp when it is done with a stage
-
-  int ti, tj;
-  if (!map_tile(p, ti, tj)) return;
-  if (p.status != nullptr && p.status->code != 0) return;  // an earlier step failed
-  const int row0 = ti * BM, col0 = tj * BN;
+  __shared__ int s_go, s_row, s_col;
+  __shared__ int s_issued;  // k-tiles whose loads have been issued
   const int KT = (p.K + kBK - 1) / kBK;
 
   const int tid = threadIdx.x;
@@ -117,6 +125,12 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
   const int g = lane >> 2, t = lane & 3;
   const int wm = warp % WARPS_M, wn = warp / WARPS_M;
 
+  if (tid == 32) {  // beside warp 0's set-up
+    int ti, tj;
+    const bool in = map_tile(p, ti, tj);
+    s_row = in ? ti * BM : -1;
+    s_col = tj * BN;
+  }
   if (tid == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -125,8 +139,13 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
       mbar_init(&empty[s], S::kThreads / 32);
     }
     fence_mbar_init();
+    s_issued = min(kStages, KT);
+    // an earlier step failed: the CTA takes one thread's reading
+    s_go = p.status == nullptr || ((volatile DevStatus*)p.status)->code == 0;
   }
   __syncthreads();
+  if (!s_go || s_row < 0) return;
+  const int row0 = s_row, col0 = s_col;
 
   auto issue = [&](int kt) {
     const int s = kt % kStages;
@@ -146,12 +165,8 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
       for (int b = 0; b < BN / 16; ++b) tma_load_2d(sB + b * 256, &tmB, &full[s], col0 + 16 * b, kt * kBK);
     }
   };
-
-  int issued = 0;  // k-tiles whose loads thread 0 has issued
-  if (tid == 0) {
+  if (tid == 0)
     for (int kt = 0; kt < kStages && kt < KT; ++kt) issue(kt);
-    issued = min(kStages, KT);
-  }
   // Pull this tile of C into L2 while the main loop runs, so the epilogue's
   // read-modify-write does not wait on HBM (one bulk prefetch per column).
   if (p.beta != 0.0 && p.cvec) {
@@ -164,9 +179,9 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
     }
   }
 
-  double acc[4][4][4];
+  double acc[MI][4][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -175,22 +190,23 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
   bool ok = true;
   for (int kt = 0; kt < KT; ++kt) {
     const int s = kt % kStages;
-    const uint32_t parity = (kt / kStages) & 1;
+    const uint32_t parity = (uint32_t)(kt / kStages) & 1u;
     // warp-uniform outcome: the DMMAs below need the whole warp converged
-    ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(&full[s], parity));
+    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[s], parity));
+    if (!ok) break;
     const double* sA = reinterpret_cast<const double*>(smem + s * S::kStageBytes);
     const double* sB = sA + BM * kBK;
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
-      double af[4][4], bf[4][2];
+      double af[MI][4], bf[4][2];
       const int ke = ks * 8 + 2 * t;  // physical k pair (ke, ke+1)
       if (AK) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < MI; ++i) {
           // the same row interleaving as for MN-major A (a thread's rows 2g, 2g + 1
           // are adjacent, for the 16-byte epilogue); its even rows meet two to a
           // bank, which the DMMA pipe hides
-          const int r0 = wm * 64 + (i >> 1) * 32 + 2 * g + (i & 1);
+          const int r0 = wm * 16 * MI + (i >> 1) * 32 + 2 * g + (i & 1);
           const int r1 = r0 + 16;
           const int ch = ks * 4 + t;
           const double2 v0 = *reinterpret_cast<const double2*>(sA + r0 * 16 + ((ch ^ (r0 & 7)) << 1));
@@ -198,11 +214,11 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
           af[i][0] = v0.x; af[i][2] = v0.y; af[i][1] = v1.x; af[i][3] = v1.y;
         }
       } else {
-        // box (wm * 64 + pr * 32) / 16 (+1 for rows +16), chunk g of rows ke, ke + 1
+        // boxes wm * MI + 2 pr and + 1 (rows +16), chunk g of rows ke, ke + 1
         const int c0 = (g ^ (ke & 7)) << 1, c1 = (g ^ ((ke + 1) & 7)) << 1;
 #pragma unroll
-        for (int pr = 0; pr < 2; ++pr) {
-          const double* bx = sA + (wm * 4 + pr * 2) * 256;
+        for (int pr = 0; pr < MI / 2; ++pr) {
+          const double* bx = sA + (wm * MI + 2 * pr) * 256;
           const double2 v00 = *reinterpret_cast<const double2*>(bx + ke * 16 + c0);
           const double2 v01 = *reinterpret_cast<const double2*>(bx + (ke + 1) * 16 + c1);
           const double2 v10 = *reinterpret_cast<const double2*>(bx + 256 + ke * 16 + c0);
@@ -231,7 +247,7 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
         }
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) dmma_16x8x8(acc[i][j], af[i], bf[j]);
     }
@@ -248,12 +264,14 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
       mbar_arrive(&empty[s]);
     }
     if (warp == 0 && kt + kStages < KT) {
-      ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(&empty[s], parity));
-      if (ok && lane == 0) issue(kt + kStages);
-      if (ok) issued = kt + kStages + 1;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], parity));
+      if (!ok) break;
+      if (lane == 0) {
+        issue(kt + kStages);
+        s_issued = kt + kStages + 1;
+      }
       __syncwarp();
     }
-    if (!ok) break;
   }
 
   // a warp that gave up (bounded wait) leaves early; all meet here
@@ -261,21 +279,20 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
     if (tid == 0) {
       set_status(p.status, kTimeout, 100);
       // Drain copies still in flight before the CTA's shared memory goes away.
-      for (int r = max(0, issued - kStages); r < issued; ++r)
-        (void)mbar_wait_bounded(&full[r % kStages], (r / kStages) & 1);
+      for (int r = max(0, s_issued - kStages); r < s_issued; ++r)
+        (void)mbar_wait_bounded(&full[r % kStages], (uint32_t)(r / kStages) & 1u);
     }
     __syncthreads();
     return;
   }
 
   // Epilogue: C = alpha * acc + beta * C on the valid (and triangle) region.
-  // C is read in groups of eight 16-byte (sixteen 8-byte) loads per thread, all
-  // in flight before the first is used: with a test around each load they ran
-  // one after the other, 27 K cycles per tile against 31 K for the main loop
-  // at K = 128 (two CTAs on the SM).
+  // A thread's loads of a group are all in flight before the first is used:
+  // with a test around each load they ran one after the other, 27 K cycles per
+  // tile against 31 K for the main loop at K = 128 (two CTAs on the SM).
   const double alpha = p.alpha, beta = p.beta;
   auto row_of = [&](int i, int r) -> int {
-    return row0 + wm * 64 + (i >> 1) * 32 + 2 * g + (i & 1) + ((r >= 2) ? 16 : 0);
+    return row0 + wm * 16 * MI + (i >> 1) * 32 + 2 * g + (i & 1) + ((r >= 2) ? 16 : 0);
   };
   auto col_of = [&](int j, int r) -> int {
     const int c = 2 * t + (r & 1);
@@ -288,80 +305,52 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (WARPS_M * WARPS_N <= 
     if (p.tri == 2 && row > col) return false;
     return true;
   };
-  // tiles 2pr and 2pr+1 hold rows (2g, 2g+1) -> one 16-byte access
-  const bool vec = p.cvec;
-  if (vec) {
-    // a tile wholly inside C (and its triangle) takes no test per element
-    const bool inside = row0 + BM <= p.M && col0 + BN <= p.N && !(p.tri == 1 && row0 < col0 + BN - 1) &&
-                        !(p.tri == 2 && row0 + BM - 1 > col0);
-    double* cbase = p.C + row_of(0, 0);
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {  // row pair pr = h / 2, columns tiles j = 2 (h & 1), + 1: eight loads in flight
-      const int pr = h >> 1, j0 = 2 * (h & 1);
-      double2 cc[8];
-      double* cp[8];
-      bool v0[8], v1[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int j = j0 + (e >> 2), r = e & 3;
-        const int row = row_of(2 * pr, r), col = col_of(j, r);
-        cp[e] = cbase + (long long)col * p.ldc + (row - row_of(0, 0));
-        v0[e] = inside || valid(row, col);
-        v1[e] = inside || valid(row + 1, col);
-        cc[e] = make_double2(0.0, 0.0);
-      }
-      if (beta != 0.0) {
-        if (inside) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) cc[e] = *reinterpret_cast<const double2*>(cp[e]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (v0[e]) cc[e].x = cp[e][0];
-            if (v1[e]) cc[e].y = cp[e][1];
-          }
-        }
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int j = j0 + (e >> 2), r = e & 3;
-        cc[e].x = fma(beta, cc[e].x, alpha * acc[2 * pr][j][r]);
-        cc[e].y = fma(beta, cc[e].y, alpha * acc[2 * pr + 1][j][r]);
-      }
-      if (inside) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) *reinterpret_cast<double2*>(cp[e]) = cc[e];
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (v0[e]) cp[e][0] = cc[e].x;
-          if (v1[e]) cp[e][1] = cc[e].y;
-        }
-      }
-    }
-    return;
-  }
+  double* cbase = p.C + (long long)col_of(0, 0) * p.ldc + row_of(0, 0);
+  // element (i, j, r) lies at cbase + off(i, j, r)
+  auto off = [&](int i, int j, int r) -> long long {
+    const int dc = BK ? j * 8 + (r & 1) : (j >> 1) * 16 + 2 * (r & 1) + (j & 1);
+    return (long long)dc * p.ldc + (i >> 1) * 32 + (i & 1) + ((r >= 2) ? 16 : 0);
+  };
+  // a tile wholly inside C (and its triangle) takes no test per element; the
+  // row tiles 2 pr and 2 pr + 1 hold rows (2g, 2g + 1): one 16-byte access
   const bool inside = row0 + BM <= p.M && col0 + BN <= p.N && !(p.tri == 1 && row0 < col0 + BN - 1) &&
                       !(p.tri == 2 && row0 + BM - 1 > col0);
+  if (inside && p.cvec) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {  // sixteen loads in flight
-    double cc[4][4];
+    for (int pr = 0; pr < MI / 2; ++pr)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < 4; ++j) {
+        double2 cc[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int row = row_of(i, r), col = col_of(j, r);
-        cc[j][r] = beta != 0.0 && (inside || valid(row, col)) ? p.C[(long long)col * p.ldc + row] : 0.0;
+        for (int r = 0; r < 4; ++r)
+          cc[r] = beta != 0.0 ? *reinterpret_cast<const double2*>(cbase + off(2 * pr, j, r)) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          cc[r].x = fma(beta, cc[r].x, alpha * acc[2 * pr][j][r]);
+          cc[r].y = fma(beta, cc[r].y, alpha * acc[2 * pr + 1][j][r]);
+          *reinterpret_cast<double2*>(cbase + off(2 * pr, j, r)) = cc[r];
+        }
       }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int row = row_of(i, r), col = col_of(j, r);
-        cc[j][r] = beta != 0.0 ? fma(beta, cc[j][r], alpha * acc[i][j][r]) : alpha * acc[i][j][r];
-        if (inside || valid(row, col)) p.C[(long long)col * p.ldc + row] = cc[j][r];
-      }
+    return;
   }
+#pragma unroll
+  for (int pr = 0; pr < MI / 2; ++pr)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      double c0[4], c1[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        c0[r] = beta != 0.0 && valid(row_of(2 * pr, r), col_of(j, r)) ? cbase[off(2 * pr, j, r)] : 0.0;
+        c1[r] = beta != 0.0 && valid(row_of(2 * pr + 1, r), col_of(j, r)) ? cbase[off(2 * pr + 1, j, r)] : 0.0;
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (valid(row_of(2 * pr, r), col_of(j, r)))
+          cbase[off(2 * pr, j, r)] = fma(beta, c0[r], alpha * acc[2 * pr][j][r]);
+        if (valid(row_of(2 * pr + 1, r), col_of(j, r)))
+          cbase[off(2 * pr + 1, j, r)] = fma(beta, c1[r], alpha * acc[2 * pr + 1][j][r]);
+      }
+    }
 }
 
 }  // namespace egpu

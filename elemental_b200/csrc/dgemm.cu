@@ -78,186 +78,202 @@ static cudaError_t launch_variant(cudaStream_t st, const CUtensorMap& ma, const 
 
 
 // ---- small products ------------------------------------------------------
-// A product with only a few 128 x 64 tiles (a panel multiply or the next
-// block column's update of a small factorization) leaves most of the GPU
-// idle and is bound by the per-SM DMMA rate of the few CTAs it has.  This form spreads it over many more warps: each warp computes a
-// 32 x 32 tile of C (2 x 4 DMMA m16n8k8 tiles) straight from global memory
-// (L2), 16 k at a time with the next 16 in flight, and a CTA of WM x WN
-// warps covers a (32 WM) x (32 WN) tile.  All of a CTA's loads come before a
-// CTA barrier and its stores after it, so C may alias A when the CTA covers
-// every column of C (WN * 32 >= N), or B when it covers every row.
+// A product with few tiles (a panel multiply or the next block column's update
+// of a small factorization) is bound by latencies, not by the DMMA rate: the
+// engine's 128 x 64 x 128 tile takes 8 us on one SM however idle the rest is.
+// Here a CTA of eight warps takes a small tile of C (32 x 32, or 16 or 32 rows
+// by all columns, or all rows by 16 columns) with the whole of K: A's and B's
+// parts are copied to shared memory by 16-byte cp.async, all in flight at
+// once together with the tile of C, so the chain is one round trip to L2, the
+// products and the store.  C may be A when the CTA covers every column of C,
+// or B when it covers every row: all of it is in shared memory before any
+// store.  (Warps that read their operands from L2 sixteen k at a time, one
+// round trip each: 22 us per launch at M = 2048, N = K = 128; now 8 to 10.)
 struct SmallParams {
   const double* A;
   const double* B;
   double* C;
   long long lda, ldb, ldc;
-  int M, N, K, tri, wm, wn;
+  int M, N, K, tri;
   double alpha, beta;
   const DevStatus* status;
 };
 
-template <bool AK, bool BK>
-__global__ void __launch_bounds__(128) dgemm_small_kernel(const SmallParams p) {
+// 16-byte cp.async of which the first `bytes` are read and the rest is zero
+__device__ __forceinline__ void cp_async16_zfill(void* smem_dst, const void* gmem_src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(bytes)
+               : "memory");
+}
+
+constexpr int small_ld(int tile) { return tile + 4; }  // MN-major parts: 4 mod 16, conflict-free fragment loads
+
+// Copy rows [r0, r0 + T) of an operand, k in [0, KP) (zero past R rows and K),
+// to shared memory: MN-major as [k][T + 4], K-major as [row][KP + 4].
+template <bool KM, int T>
+__device__ __forceinline__ void small_stage(double* S, const double* G, long long ld, int r0, int R, int K, int KP) {
+  if (!KM) {
+    constexpr int CH = T / 2;  // chunks per k
+    for (int e = threadIdx.x; e < KP * CH; e += 256) {
+      const int k = e / CH, r = 2 * (e % CH), left = R - (r0 + r);
+      const int bytes = k < K ? (left >= 2 ? 16 : left == 1 ? 8 : 0) : 0;
+      cp_async16_zfill(S + k * small_ld(T) + r, bytes ? G + (long long)k * ld + r0 + r : G, bytes);
+    }
+  } else {
+    const int ch = KP / 2, lds = KP + 4;
+    for (int e = threadIdx.x; e < T * ch; e += 256) {
+      const int r = e / ch, k = 2 * (e - r * ch), left = K - k;
+      const int bytes = r0 + r < R ? (left >= 2 ? 16 : left == 1 ? 8 : 0) : 0;
+      cp_async16_zfill(S + r * lds + k, bytes ? G + (long long)(r0 + r) * ld + k : G, bytes);
+    }
+  }
+}
+
+template <bool AK, bool BK, int TM, int TN>
+__global__ void __launch_bounds__(256) dgemm_small_kernel(const SmallParams p) {
+  extern __shared__ __align__(16) double ss[];
+  constexpr int TILES = (TM / 16) * (TN / 8), PER = TILES / 8;  // 16 x 8 DMMA tiles per warp
+  static_assert(TILES % 8 == 0, "eight warps");
   if (p.status != nullptr && p.status->code != 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int row0 = (blockIdx.x * p.wm + warp % p.wm) * 32;
-  const int col0 = (blockIdx.y * p.wn + warp / p.wm) * 32;
-  // a warp whose tile is wholly outside C or outside the triangle has no work
-  // but still meets the CTA barrier
-  const bool live = row0 < p.M && col0 < p.N && !(p.tri == 1 && row0 + 31 < col0) && !(p.tri == 2 && row0 > col0 + 31);
-  double acc[2][4][4];
+  const int row0 = blockIdx.x * TM, col0 = blockIdx.y * TN;
+  if ((p.tri == 1 && row0 + TM - 1 < col0) || (p.tri == 2 && row0 > col0 + TN - 1)) return;
+  const int KP = (p.K + 7) & ~7;
+  double* sA = ss;
+  double* sB = ss + (AK ? TM * (KP + 4) : KP * small_ld(TM));
+  small_stage<AK, TM>(sA, p.A, p.lda, row0, p.M, p.K, KP);
+  small_stage<BK, TN>(sB, p.B, p.ldb, col0, p.N, p.K, KP);
+  // this warp's tiles: row tile rt, column tiles ct, ct + 1, ..
+  const int rt = (warp * PER) / (TN / 8), ct = (warp * PER) % (TN / 8);
+  double acc[PER][4], cc[PER][4];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < PER; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
-  if (live) {
-    // this lane's rows of op(A) and columns of op(B), clamped (a row or column
-    // past the edge is read at a valid address and multiplied by zero)
-    const double* ar[4];
-    const double* bc[4];
-    bool am[4], bm[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {  // rows row0 + g + 8 q
-      const int m = row0 + g + 8 * q;
-      am[q] = m < p.M;
-      ar[q] = p.A + (AK ? (long long)min(m, p.M - 1) * p.lda : (long long)min(m, p.M - 1));
+    for (int r = 0; r < 4; ++r) {
+      const int m = row0 + 16 * rt + g + (r >= 2 ? 8 : 0), n = col0 + 8 * (ct + j) + 2 * t + (r & 1);
+      const bool v = p.beta != 0.0 && m < p.M && n < p.N && !(p.tri == 1 && m < n) && !(p.tri == 2 && m > n);
+      cc[j][r] = v ? p.C[m + (long long)n * p.ldc] : 0.0;
+      acc[j][r] = 0.0;
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = col0 + 8 * j + g;
-      bm[j] = n < p.N;
-      bc[j] = p.B + (BK ? (long long)min(n, p.N - 1) * p.ldb : (long long)min(n, p.N - 1));
-    }
-    const long long as = AK ? 1 : p.lda, bs = BK ? 1 : p.ldb;  // k stride
-    double af[4][4], bf[4][4];  // [k offset t, t+4, t+8, t+12][row / column slot]
-    double an[4][4], bn[4][4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = t + 4 * u;
-      const bool kin = k < p.K;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) af[u][q] = (kin && am[q]) ? __ldg(ar[q] + k * as) : 0.0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bf[u][j] = (kin && bm[j]) ? __ldg(bc[j] + k * bs) : 0.0;
-    }
-    for (int k0 = 0; k0 < p.K; k0 += 16) {
-      const bool more = k0 + 16 < p.K;
-      if (more) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int k = k0 + 16 + t + 4 * u;
-          const bool kin = k < p.K;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) an[u][q] = (kin && am[q]) ? __ldg(ar[q] + k * as) : 0.0;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) bn[u][j] = (kin && bm[j]) ? __ldg(bc[j] + k * bs) : 0.0;
-        }
-      }
-      // two k8 steps: k = k0 + {t, t+4} and k0 + 8 + {t, t+4}
-#pragma unroll
-      for (int s2 = 0; s2 < 2; ++s2) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          // rows 16 i + g (slot 2 i) and 16 i + g + 8 (slot 2 i + 1)
-          const double a4[4] = {af[2 * s2][2 * i], af[2 * s2][2 * i + 1], af[2 * s2 + 1][2 * i],
-                                af[2 * s2 + 1][2 * i + 1]};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const double b2[2] = {bf[2 * s2][j], bf[2 * s2 + 1][j]};
-            dmma_16x8x8(acc[i][j], a4, b2);
-          }
-        }
-      }
-      if (more) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            af[u][q] = an[u][q];
-            bf[u][q] = bn[u][q];
-          }
-      }
-    }
-  }
-  // every load of the CTA is done before any store (C may alias A or B)
+  cp_async_wait_all();
   __syncthreads();
-  if (!live) return;
-  // all of the tile's C loads in flight before the first is used
-  double cc[2][4][4];
+  const int as = AK ? 1 : small_ld(TM), am = AK ? KP + 4 : 1;  // k and row strides
+  const int bs = BK ? 1 : small_ld(TN), bn = BK ? KP + 4 : 1;
+  const double* pa = sA + (16 * rt + g) * am + t * as;
+  const double* pb = sB + (8 * ct + g) * bn + t * bs;
+  double acc2[PER][4];  // two chains per tile
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < PER; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int r = 0; r < 4; ++r) acc2[j][r] = 0.0;
+  auto step = [&](double (&d)[PER][4], int k0) {
+    const double a[4] = {pa[k0 * as], pa[k0 * as + 8 * am], pa[(k0 + 4) * as], pa[(k0 + 4) * as + 8 * am]};
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int m = row0 + 16 * i + g + (r >= 2 ? 8 : 0), n = col0 + 8 * j + 2 * t + (r & 1);
-        const bool v = p.beta != 0.0 && m < p.M && n < p.N && !(p.tri == 1 && m < n) && !(p.tri == 2 && m > n);
-        cc[i][j][r] = v ? p.C[m + (long long)n * p.ldc] : 0.0;
-      }
+    for (int j = 0; j < PER; ++j) {
+      const double b[2] = {pb[k0 * bs + 8 * j * bn], pb[(k0 + 4) * bs + 8 * j * bn]};
+      dmma_16x8x8(d[j], a, b);
+    }
+  };
+  int k0 = 0;
+#pragma unroll 2
+  for (; k0 + 8 < KP; k0 += 16) {
+    step(acc, k0);
+    step(acc2, k0 + 8);
+  }
+  if (k0 < KP) step(acc, k0);
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < PER; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int m = row0 + 16 * i + g + (r >= 2 ? 8 : 0), n = col0 + 8 * j + 2 * t + (r & 1);
-        const bool v = m < p.M && n < p.N && !(p.tri == 1 && m < n) && !(p.tri == 2 && m > n);
-        const double x = p.beta == 0.0 ? p.alpha * acc[i][j][r] : fma(p.beta, cc[i][j][r], p.alpha * acc[i][j][r]);
-        if (v) p.C[m + (long long)n * p.ldc] = x;
-      }
+    for (int r = 0; r < 4; ++r) {
+      const int m = row0 + 16 * rt + g + (r >= 2 ? 8 : 0), n = col0 + 8 * (ct + j) + 2 * t + (r & 1);
+      const bool v = m < p.M && n < p.N && !(p.tri == 1 && m < n) && !(p.tri == 2 && m > n);
+      const double x = acc[j][r] + acc2[j][r];
+      if (v) p.C[m + (long long)n * p.ldc] = p.beta == 0.0 ? p.alpha * x : fma(p.beta, cc[j][r], p.alpha * x);
+    }
 }
 
-// Byte ranges [lo, hi) of a column-major view (rows x cols, ld) in memory.
+template <bool AK, bool BK, int TM, int TN>
+static cudaError_t launch_small_variant(cudaStream_t st, const SmallParams& p) {
+  auto kern = dgemm_small_kernel<AK, BK, TM, TN>;
+  constexpr int kMax = 200 * 1024;
+  static unsigned attr_mask = 0;  // per template instance, one bit per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 32 || !(attr_mask & (1u << dev))) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMax);
+    if (e != cudaSuccess) return e;
+    if (dev < 32) attr_mask |= (1u << dev);
+  }
+  const int KP = (p.K + 7) & ~7;
+  const size_t smem = sizeof(double) * ((size_t)(AK ? TM * (KP + 4) : KP * small_ld(TM)) +
+                                        (size_t)(BK ? TN * (KP + 4) : KP * small_ld(TN)));
+  if (smem > kMax) return cudaErrorInvalidValue;
+  const dim3 grid((p.M + TM - 1) / TM, (p.N + TN - 1) / TN);
+  kern<<<grid, 256, smem, st>>>(p);
+  count_launch();
+  return cudaGetLastError();
+}
+
+template <int TM, int TN>
+static cudaError_t launch_small_tile(cudaStream_t st, bool ak, bool bk, const SmallParams& p) {
+  if (ak && bk) return launch_small_variant<true, true, TM, TN>(st, p);
+  if (ak) return launch_small_variant<true, false, TM, TN>(st, p);
+  if (bk) return launch_small_variant<false, true, TM, TN>(st, p);
+  return launch_small_variant<false, false, TM, TN>(st, p);
+}
+
+// Do two column-major views share an element?  Views with the same leading
+// dimension are compared as blocks of one matrix (a panel's row block and the
+// block below it interleave in memory without sharing anything); others by the
+// memory they span.
 static bool views_overlap(const double* a, long long rows_a, long long cols_a, long long lda, const double* b,
                           long long rows_b, long long cols_b, long long ldb) {
+  const intptr_t bytes = reinterpret_cast<intptr_t>(a) - reinterpret_cast<intptr_t>(b);
+  if (lda == ldb && bytes % 8 == 0 && rows_a <= lda && rows_b <= ldb) {
+    const long long diff = bytes / 8, dc = diff >= 0 ? diff / lda : -((-diff + lda - 1) / lda), dr = diff - dc * lda;
+    // a's element (0, 0) is b's (dr, dc), 0 <= dr < ld; its rows past the end
+    // of b's column are those of (dr - ld, dc + 1)
+    auto meet = [&](long long r, long long c) { return r < rows_b && r + rows_a > 0 && c < cols_b && c + cols_a > 0; };
+    return meet(dr, dc) || meet(dr - lda, dc + 1);
+  }
   const uintptr_t a0 = reinterpret_cast<uintptr_t>(a), a1 = a0 + 8 * ((cols_a - 1) * lda + rows_a);
   const uintptr_t b0 = reinterpret_cast<uintptr_t>(b), b1 = b0 + 8 * ((cols_b - 1) * ldb + rows_b);
   return a0 < b1 && b0 < a1;
 }
 
-// The small form when the 128 x 64 tiles would not fill the SMs; returns
-// EGPU_ERR_UNSUPPORTED when it does not apply (then the TMA engine runs).
+// The small form when it applies; else EGPU_ERR_UNSUPPORTED (then the TMA
+// engine runs).
 static int launch_dgemm_small(cudaStream_t st, bool a_kmajor, bool b_kmajor, int M, int N, int K, double alpha,
                               const double* A, long long lda, const double* B, long long ldb, double beta, double* C,
                               long long ldc, int tri, DevStatus* status) {
-  // only the smallest products (at most 40 of the engine's tiles, K <= 256):
-  // between that and a full wave the TMA engine measured as fast or faster
-  const long long big_tiles = (long long)((M + 127) / 128) * ((N + 63) / 64);
-  if (big_tiles > 40 || K > 256) return EGPU_ERR_UNSUPPORTED;
+  if (K > 256) return EGPU_ERR_UNSUPPORTED;
   const bool alias_a = views_overlap(C, M, N, ldc, A, a_kmajor ? K : M, a_kmajor ? M : K, lda);
   const bool alias_b = views_overlap(C, M, N, ldc, B, b_kmajor ? K : N, b_kmajor ? N : K, ldb);
-  int wm = 2, wn = 2;
   if (alias_a && alias_b) return EGPU_ERR_UNSUPPORTED;
   // in place only as the drivers use it: C is A (the same rows) or C is B
   // (column n of C is column n of op(B)^T)
-  if (alias_a && !(C == A && ldc == lda && !a_kmajor)) return EGPU_ERR_UNSUPPORTED;
-  if (alias_b && !(C == B && ldc == ldb && b_kmajor)) return EGPU_ERR_UNSUPPORTED;
-  if (alias_a) {  // every column of C in one CTA
-    if (N > 128) return EGPU_ERR_UNSUPPORTED;
-    wn = (N + 31) / 32;
-    wm = std::max(1, 4 / wn);
-  } else if (alias_b) {  // every row of C in one CTA
-    if (M > 128) return EGPU_ERR_UNSUPPORTED;
-    wm = (M + 31) / 32;
-    wn = std::max(1, 4 / wm);
-  }
+  if (alias_a && !(C == A && ldc == lda && !a_kmajor && N <= 128 && K <= 128)) return EGPU_ERR_UNSUPPORTED;
+  if (alias_b && !(C == B && ldc == ldb && b_kmajor && M <= 128 && K <= 128)) return EGPU_ERR_UNSUPPORTED;
+  const long long t32 = (long long)((M + 31) / 32) * ((N + 31) / 32);
+  // where the engine, whose tiles need half the operand traffic, catches up (K =
+  // 128, us, engine / this form): 1600 tiles of 32 x 32 (1280^2) 28.9 / 22.8,
+  // 2304 tiles (1536^2) 28.9 / 30.9; in place one wave of CTAs (M = 2048: 22 /
+  // 10; the Cholesky at n = 16384 0.6% slower with the whole range of M here)
+  if (!alias_a && !alias_b && t32 / (tri ? 2 : 1) > 1480) return EGPU_ERR_UNSUPPORTED;
+  if (alias_a && M > 32 * 148) return EGPU_ERR_UNSUPPORTED;
+  if (alias_b && N > 32 * 148) return EGPU_ERR_UNSUPPORTED;
   SmallParams p;
   p.A = A; p.B = B; p.C = C; p.lda = lda; p.ldb = ldb; p.ldc = ldc;
-  p.M = M; p.N = N; p.K = K; p.tri = tri; p.wm = wm; p.wn = wn; p.alpha = alpha; p.beta = beta; p.status = status;
-  const dim3 grid((M + 32 * wm - 1) / (32 * wm), (N + 32 * wn - 1) / (32 * wn));
+  p.M = M; p.N = N; p.K = K; p.tri = tri; p.alpha = alpha; p.beta = beta; p.status = status;
   const double lo_n = std::min(M, N), rect = tri == 1 ? std::max(0, M - N) : std::max(0, N - M);
   const double entries = tri == 0 ? (double)M * N : lo_n * (lo_n + 1) / 2 + rect * lo_n;
   TraceMark tm(st, beta == 0.0 ? kTraceTrsm : kTraceUpdate, 2.0 * entries * K,
                8.0 * ((double)M * K + (double)N * K + (beta == 0.0 ? 1.0 : 2.0) * entries));
-  if (a_kmajor && b_kmajor) dgemm_small_kernel<true, true><<<grid, 32 * wm * wn, 0, st>>>(p);
-  else if (a_kmajor) dgemm_small_kernel<true, false><<<grid, 32 * wm * wn, 0, st>>>(p);
-  else if (b_kmajor) dgemm_small_kernel<false, true><<<grid, 32 * wm * wn, 0, st>>>(p);
-  else dgemm_small_kernel<false, false><<<grid, 32 * wm * wn, 0, st>>>(p);
-  count_launch();
-  const cudaError_t e = cudaGetLastError();
+  cudaError_t e;
+  if (alias_a && M <= 16 * 148) e = launch_small_tile<16, 128>(st, a_kmajor, b_kmajor, p);
+  else if (alias_a) e = launch_small_tile<32, 128>(st, a_kmajor, b_kmajor, p);
+  else if (alias_b) e = launch_small_tile<128, 16>(st, a_kmajor, b_kmajor, p);
+  else e = launch_small_tile<32, 32>(st, a_kmajor, b_kmajor, p);
   if (e != cudaSuccess) {
     set_last_error(e, "dgemm_small launch", __FILE__, __LINE__);
     return EGPU_ERR_CUDA;

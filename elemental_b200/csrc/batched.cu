@@ -1142,6 +1142,19 @@ static int variant_prepare(const Variant& v, int kind, int* per_sm) {
   return EGPU_OK;
 }
 
+// The shape used without tuning, from the kind and the largest order.  FP64 HPD:
+// two CTAs per SM with 16-wide panels, whose chains overlap (4096 systems, n =
+// 32..512: 9.9 ms against 11.2 with one CTA and 32-wide panels; n = 512 alone
+// 3.99 and 4.03).  FP64 GE: the same with 128 threads while the systems are
+// small (n <= 256: 5.7 against 6.6 ms; n <= 64 1.06 and 1.87), above that one CTA
+// with 32-wide panels, which moves the trailing matrix half as often (what the
+// autotuner picks at n = 512 too).
+static int default_variant(int kind, int precision, int nmax) {
+  if (precision != 0) return 0;
+  if (kind == 0) return 1;
+  return nmax <= 256 ? 2 : 0;
+}
+
 static void sort_items(std::vector<BatchItem>& items) {
   std::stable_sort(items.begin(), items.end(), [](const BatchItem& a, const BatchItem& b) { return a.n > b.n; });
 }
@@ -1172,10 +1185,10 @@ int egpu_batched_launch(int kind, cudaStream_t st, int sm_count, int count, cons
     items[i].id = i;
   }
   sort_items(items);
-  const Variant& v = kVariants[0][0];
+  const Variant& v = kVariants[0][default_variant(kind, 0, count > 0 ? items[0].n : 0)];
   int per_sm = 1;
   BTRY(variant_prepare(v, kind, &per_sm));
-  const int grid = std::max(1, std::min(sm_count, count));
+  const int grid = std::max(1, std::min(std::min(per_sm, 2) * sm_count, count));
   unsigned char* base = static_cast<unsigned char*>(ws);
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -1187,7 +1200,7 @@ int egpu_batched_launch(int kind, cudaStream_t st, int sm_count, int count, cons
   BatchItem* d_items = static_cast<BatchItem*>(take(sizeof(BatchItem) * std::max(count, 1)));
   int* d_counter = static_cast<int*>(take(sizeof(int)));
   int* d_info = static_cast<int*>(take(sizeof(int) * std::max(count, 1)));
-  double* d_scr = static_cast<double*>(take(sizeof(double) * (size_t)sm_count * kScrDoubles));
+  double* d_scr = static_cast<double*>(take(sizeof(double) * (size_t)std::min(2 * sm_count, std::max(count, 1)) * kScrDoubles));
   if (off > ws_bytes) return EGPU_ERR_ALLOC;
   if (count == 0) return EGPU_OK;
   EGPU_CUDA_TRY(cudaMemcpyAsync(d_items, items.data(), sizeof(BatchItem) * count, cudaMemcpyHostToDevice, st));
@@ -1208,7 +1221,7 @@ int egpu_batched_launch(int kind, cudaStream_t st, int sm_count, int count, cons
 
 size_t egpu_batched_ws_bytes(int count, int sm_count) {
   return sizeof(BatchItem) * (size_t)std::max(count, 1) + sizeof(int) * (size_t)std::max(count, 1) + 4096 +
-         sizeof(double) * (size_t)sm_count * kScrDoubles;
+         sizeof(double) * (size_t)std::min(2 * sm_count, std::max(count, 1)) * kScrDoubles;
 }
 
 // ---------------------------------------------------------------------------
@@ -1240,10 +1253,10 @@ static int plan_default_shape(BatchPlan* p) {
   p->nclass = 1;
   p->cbeg[0] = 0;
   p->cend[0] = p->count;
-  p->cvar[0] = 0;
+  p->cvar[0] = default_variant(p->kind, p->precision, p->count > 0 ? p->items[0].n : 0);
   p->cnmax[0] = kBmaxN;
   int per_sm = 1;
-  BTRY(variant_prepare(kVariants[p->precision][0], p->kind, &per_sm));
+  BTRY(variant_prepare(kVariants[p->precision][p->cvar[0]], p->kind, &per_sm));
   p->cgrid[0] = per_sm * p->sm_count;
   return EGPU_OK;
 }

@@ -48,6 +48,7 @@ constexpr int kTsConsumers = 256;              // 8 warps: warp w owns rows 16w 
 constexpr int kTsThreads = kTsConsumers + 32;  // + the producer warp
 constexpr int kTsKC = 32;                      // k chunk
 constexpr int kTsMaxRhs = 64;
+constexpr int kTsMaxGroups = 8;
 // A ring stage holds an A chunk (amode 0: [a + kl*(hs+4)], amode 1:
 // [kl + a*36]) and an X chunk ([kl + c*36]); both pitches are 4 mod 16
 // (conflict-free 8-byte fragment loads) and every stage starts on a
@@ -71,6 +72,8 @@ struct TsParams {
   int n, nrhs, nb, nblk, bwd, amode;
   int mode;        // 0 plain, 1 column-prescaled, 2 row-prescaled
   int strips, hs;  // tasks per block row and their height
+  int groups, gw, gsz;  // groups of right-hand sides, columns and CTAs per group
+  int bid;              // this CTA's number in its group (set by the kernel)
   int* flags;
   int epoch;
   DevStatus* status;
@@ -163,7 +166,7 @@ __device__ void ts_producer(const CUtensorMap* mapL, const CUtensorMap* mapW, co
     tma_prefetch_desc(mapW);
   }
   int gq = 0;  // chunks of this CTA so far
-  for (int task = blockIdx.x; task < p.nblk * p.strips; task += gridDim.x) {
+  for (int task = p.bid; task < p.nblk * p.strips; task += p.gsz) {
     const TsTask t = ts_task(p, task);
     if (t.mr <= 0) continue;
     const int Q = (t.s + 1) * cpp;
@@ -251,7 +254,7 @@ __device__ void ts_consumers(const TsParams& p, double* sm, uint64_t* fullA, uin
   const int cpp = (p.nb + kTsKC - 1) / kTsKC;
   const int ldA = p.amode == 0 ? p.hs + 4 : kTsCT;  // A stage pitch
   int gq = 0;
-  for (int task = blockIdx.x; task < p.nblk * p.strips; task += gridDim.x) {
+  for (int task = p.bid; task < p.nblk * p.strips; task += p.gsz) {
     const TsTask t = ts_task(p, task);
     double acc[NT][4];
 #pragma unroll
@@ -368,7 +371,16 @@ __device__ void ts_consumers(const TsParams& p, double* sm, uint64_t* fullA, uin
 template <int NT>
 __global__ void __launch_bounds__(kTsThreads, 1) trsm_skinny_kernel(const __grid_constant__ CUtensorMap mapL,
                                                                     const __grid_constant__ CUtensorMap mapW,
-                                                                    TsParams p) {
+                                                                    const TsParams pp) {
+  // this CTA's group of right-hand sides: its columns, its counters
+  TsParams p = pp;
+  const int grp = (int)blockIdx.x / pp.gsz;
+  p.bid = (int)blockIdx.x - grp * pp.gsz;
+  if (pp.groups > 1) {
+    p.X += (long long)grp * pp.gw * pp.ldx;
+    p.nrhs = min(pp.gw, pp.nrhs - grp * pp.gw);
+    p.flags += grp * pp.nblk;
+  }
   // TMA boxes land at stage starts: the dynamic region must be 128-byte
   // aligned (it follows the static barriers)
   extern __shared__ __align__(128) double sm[];
@@ -395,9 +407,11 @@ __global__ void __launch_bounds__(kTsThreads, 1) trsm_skinny_kernel(const __grid
   else ts_consumers<NT>(p, sm, fullA, fullX, empty);
 }
 
-size_t trsm_skinny_flag_bytes(int n, int nb) { return sizeof(int) * (size_t)((n + nb - 1) / nb) + 256; }
+size_t trsm_skinny_flag_bytes(int n, int nb) {
+  return sizeof(int) * (size_t)((n + nb - 1) / nb) * kTsMaxGroups + 256;
+}
 
-// flags: device array of ceil(n/nb) arrival counters, zero before the first
+// flags: device array (trsm_skinny_flag_bytes) of arrival counters, zero before the first
 // sweep of a sequence; sweep number `epoch` (1, 2, ...) of the sequence
 // waits for counters to reach strips x epoch.
 int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, const double* L, long long lda,
@@ -427,7 +441,23 @@ int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, con
       !make_tma_2d(&mapW, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, Winv, nb, (uint64_t)p.nblk * nb, 8ull * nb, bi, bo,
                    false))
     return EGPU_ERR_UNSUPPORTED;
+  // Right-hand sides are independent, and a step of the chain is as long as
+  // its products: the plain form gives groups of columns to their own CTAs
+  // (the triangle is then read once per group).  Groups of 8 while a CTA then
+  // has at most four block rows, which it must catch up with one after the
+  // other, else of 16.  Both sweeps of a Cholesky solve, us, one group / groups
+  // of 16 / of 8: n = 2048, 64 right-hand sides 838 / 354 / 286, n = 8192, 32
+  // 1864 / 1248 / 957, n = 16384, 64 6425 / 3015 / 3767.
+  p.groups = 1;
+  p.gw = nrhs;
+  if (p.mode == 0 && nrhs > 8) {
+    p.gw = (long long)((nrhs + 7) / 8) * p.nblk <= 4ll * sm_count ? 8 : 16;
+    p.groups = (nrhs + p.gw - 1) / p.gw;
+  }
+  p.gsz = std::min(p.nblk * p.strips, std::max(1, sm_count / p.groups));
+  p.bid = 0;
   const size_t smem = sizeof(double) * kTsSmemDoubles;
+  nrhs = std::min(nrhs, p.gw);  // columns of one CTA
   const int nt = nrhs <= 8 ? 1 : nrhs <= 16 ? 2 : nrhs <= 32 ? 4 : 8;
   void (*kern)(const CUtensorMap, const CUtensorMap, TsParams) = nt == 1   ? trsm_skinny_kernel<1>
                                                                  : nt == 2 ? trsm_skinny_kernel<2>
@@ -442,8 +472,8 @@ int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, con
     }
     attr[ai] = true;
   }
-  const int grid = std::min(p.nblk * p.strips, sm_count);
-  TraceMark tm(st, kTraceSolve, (double)n * n * nrhs, 4.0 * (double)n * n + 16.0 * n * nrhs);
+  const int grid = p.groups * p.gsz;
+  TraceMark tm(st, kTraceSolve, (double)n * n * p.nrhs, 4.0 * (double)n * n + 16.0 * n * p.nrhs);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kTsThreads);

@@ -565,19 +565,8 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
   // diagonal-block inverses by warps, then the DMMA doubling steps
   const int bb = ncols;
   double* S = sm;
-  for (int e0 = tid; e0 < bb * bb; e0 += 8 * kRpThreads) {  // .cg: rows written by other CTAs
-    double x[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = e0 + q * kRpThreads, r = e % bb, c = e / bb;
-      x[q] = (e < bb * bb && r >= c) ? __ldcg(&A[(long long)c * lda + r]) : 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = e0 + q * kRpThreads, r = e % bb, c = e / bb;
-      if (e < bb * bb && r >= c) SE(S, r, c) = x[q];
-    }
-  }
+  tri_load_async(S, A, lda, bb, false);  // rows written by other CTAs: not read through L1 before
+  cp_async_wait_all();
   __syncthreads();
   double* Xl = S + 128 * kLDS + 128;
   double* T = Xl + 8 * 16 * kLeafLD;
@@ -586,10 +575,7 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
   for (int q = warp; q < bp / 16; q += kRpThreads / 32) warp_trinv16(S, kLDS, 16 * q, 1, Xl + q * 16 * kLeafLD, kLeafLD);
   __syncthreads();
   smem_trinv_dmma(S, bp, Xl, T);
-  for (int e = tid; e < bb * bb; e += kRpThreads) {
-    const int r = e % bb, c = e / bb;
-    W[r + (long long)c * ldw] = (r > c) ? SE(S, r, c) : (r == c ? 1.0 : 0.0);
-  }
+  tri_store(S, W, ldw, bb, false, true);  // the leaves hold the unit diagonal
 }
 
 // Launch the register-resident panel when m fits one cluster (b <= m <= 16 x

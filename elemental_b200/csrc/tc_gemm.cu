@@ -8,20 +8,26 @@
 // hi*hi + hi*lo + lo*hi, which keeps ~21 bits of the FP32 product (the
 // dropped lo*lo term is 2^-22 relative).  terms = 1 is the plain TF32 product.
 //
-// Each CTA (one per SM at a time, 320 threads) takes a contiguous run of up
+// Each CTA (one per SM at a time, 576 threads) takes a contiguous run of up
 // to 8 output tiles of 128 x 128 (triangular tile lists for the symmetric
 // rank-k update of a lower triangle):
-//   warp 8 lane 0: TMA producer, 128-byte-swizzled 128 x 32 tiles into a
+//   warp 16 lane 0: TMA producer, 128-byte-swizzled 128 x 32 tiles into a
 //                  ring of stages that runs across tile boundaries
 //                  (mbarrier full/empty pairs, bounded waits);
-//   warp 9 lane 0: MMA issuer, tcgen05.mma.cta_group::1.kind::tf32 128x128x8,
+//   warp 17 lane 0: MMA issuer, tcgen05.mma.cta_group::1.kind::tf32 128x128x8,
 //                  four per 32-wide k tile and term, into one of two TMEM
 //                  accumulators (256 columns) so that a tile's epilogue
 //                  overlaps the next tile's MMAs;
-//   warps 0-7    : epilogue, C rows read into registers before the
-//                  accumulator is ready, then tcgen05.ld.32x32b of their 32
-//                  TMEM lanes (warp e: lanes 32 (e % 4).., columns 64 (e / 4)..)
-//                  and a coalesced store, one output row per thread.
+//   warps 0-15   : epilogue, two sets of 8 that take alternate tiles (set s
+//                  accumulator s): one set's C loads are in flight while the
+//                  other set stores.  A warp reads its 32 TMEM lanes
+//                  (tcgen05.ld.32x32b; warp e of a set: lanes 32 (e % 4)..,
+//                  columns 64 (e / 4)..) 32 columns at a time, one output row
+//                  per thread, coalesced; the first 32 columns of C are loaded
+//                  before the accumulator is ready, the next before the first
+//                  are stored.
+// One set left the memory idle while it stored: updates of a factorization (n = 16384, K =
+// 128) 18.6 -> 17.9 ms busy per solve.
 #include <cudaTypedefs.h>
 
 #include "internal.h"
@@ -31,9 +37,9 @@ namespace egpu {
 namespace {
 
 constexpr int kTcBM = 128, kTcBN = 128, kTcBK = 32;  // BK: 32 TF32 = one 128-byte swizzle row
-constexpr int kTcThreads = 320;  // 8 epilogue warps, producer, MMA issuer
-constexpr int kTcEpiWarps = 8;
-constexpr int kTcProdWarp = 8, kTcMmaWarp = 9;
+constexpr int kTcThreads = 576;  // two sets of 8 epilogue warps, producer, MMA issuer
+constexpr int kTcEpiWarps = 8;   // per set
+constexpr int kTcProdWarp = 16, kTcMmaWarp = 17;
 constexpr int kTcTileBytes = kTcBM * kTcBK * 4;  // 16 KiB per operand tile
 
 template <int NT>
@@ -122,7 +128,7 @@ __device__ __forceinline__ void tc_tile_of(const TcParams& p, int bid, int& tm, 
 }  // namespace
 
 template <int NT>
-__global__ void __maxnreg__(200) tc_gemm_kernel(const __grid_constant__ CUtensorMap mah,
+__global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_constant__ CUtensorMap mah,
                                                                  const __grid_constant__ CUtensorMap mbh,
                                                                  const __grid_constant__ CUtensorMap mal,
                                                                  const __grid_constant__ CUtensorMap mbl,
@@ -134,7 +140,7 @@ __global__ void __maxnreg__(200) tc_gemm_kernel(const __grid_constant__ CUtensor
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::kStages * S::kStageBytes);
   uint64_t* empty = full + S::kStages;
   uint64_t* tfull = empty + S::kStages;  // [2] accumulator ready
-  uint64_t* tempty = tfull + 2;          // [2] accumulator drained (8 epilogue warps arrive)
+  uint64_t* tempty = tfull + 2;          // [2] accumulator drained (the 8 warps of its set arrive)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -221,27 +227,27 @@ __global__ void __maxnreg__(200) tc_gemm_kernel(const __grid_constant__ CUtensor
       }
     }
   } else {
-    // ---- epilogue: warp e reads TMEM lanes 32 (e % 4) .. (its quarter) and
-    // columns 64 (e / 4) .. of each tile; each thread owns one output row.
-    const int q = warp & 3, half = warp >> 2;
-    int i = 0;
-    for (int t = t_first; t < t_end; ++t, ++i) {
+    // ---- epilogue: set `set` takes tiles set, set + 2, ..; each thread owns
+    // one output row (columns 64 half .. of the tile)
+    const int set = warp >> 3, q = warp & 3, half = (warp >> 2) & 1;
+    for (int i = set, t = t_first + set; t < t_end; t += 2, i += 2) {
       int tm, tn;
       tc_tile_of(p, t, tm, tn);
       const int m0 = tm * kTcBM, n0 = tn * kTcBN + half * 64;
       const int r = m0 + q * 32 + lane;
-      const int a = i & 1;
+      const int a = set;
       // columns n0 + j, j < jmax, of row r are written (bounds, lower triangle)
       int jmax = r < p.M ? min(64, p.N - n0) : 0;
       if (p.tri) jmax = min(jmax, r - n0 + 1);
       float* cbase = p.C + (long long)n0 * p.ldc + (r < p.M ? r : 0);
-      // this thread's 64 C entries in flight while the MMAs run
-      float cv[64];
-      {
-        const float* cp = cbase;
+      // 32 C entries of this thread at a time, in flight together
+      float cv[32];
+      auto load_c = [&](int c0) {
+        const float* cp = cbase + (long long)c0 * p.ldc;
 #pragma unroll
-        for (int j = 0; j < 64; ++j, cp += p.ldc) cv[j] = (p.beta != 0.0f && j < jmax) ? *cp : 0.0f;
-      }
+        for (int j = 0; j < 32; ++j, cp += p.ldc) cv[j] = (p.beta != 0.0f && c0 + j < jmax) ? *cp : 0.0f;
+      };
+      load_c(0);
       const bool have = __all_sync(0xffffffffu, mbar_wait_bounded(&tfull[a], (uint32_t)(i >> 1) & 1u));
       if (!have) {
         if (lane == 0) { *abort_flag = 1; set_status(p.status, kTimeout, 103); }
@@ -253,13 +259,14 @@ __global__ void __maxnreg__(200) tc_gemm_kernel(const __grid_constant__ CUtensor
       for (int c0 = 0; c0 < 64; c0 += 32) {
         float v[32];
         tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * kTcBN + half * 64 + c0), v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = c0 + j < jmax ? fmaf(p.alpha, v[j], p.beta * cv[j]) : 0.0f;
+        if (c0 == 0) load_c(32);
         float* cp;  // opaque copy of the base: keeps the load addresses from staying live
         asm volatile("mov.b64 %0, %1;" : "=l"(cp) : "l"(cbase + (long long)c0 * p.ldc));
 #pragma unroll
-        for (int j = 0; j < 32; ++j, cp += p.ldc) {
-          v[j] = c0 + j < jmax ? fmaf(p.alpha, v[j], p.beta * cv[c0 + j]) : 0.0f;
+        for (int j = 0; j < 32; ++j, cp += p.ldc)
           if (c0 + j < jmax) *cp = v[j];
-        }
         if (split && n0 + c0 < p.swidth) {  // the result's TF32 hi/lo split, 16-byte stores
           float* sh = p.sh + (long long)(r - p.srow0) * p.sldk + (n0 + c0);
           float* sl = p.sl + (long long)(r - p.srow0) * p.sldk + (n0 + c0);

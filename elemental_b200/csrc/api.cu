@@ -144,7 +144,7 @@ int potrf_seq(egpu_context* h, int uplo, int n, double* A, long long lda, double
     const int b = std::min(nb, n - k);
     const int m2 = n - k - b;
     double* A11 = A + k + (size_t)k * lda;
-    TRY(launch_potrf_diag(st, uplo, A11, lda, b, W, nb, h->dstatus, k));
+    TRY(launch_potrf_diag(st, uplo, A11, lda, b, m2 > 0 ? W : nullptr, nb, h->dstatus, k));
     if (m2 == 0) continue;
     if (uplo == EGPU_LOWER) {
       double* A21 = A + (k + b) + (size_t)k * lda;
@@ -185,7 +185,7 @@ int potrf_panel(egpu_context* h, cudaStream_t st, int uplo, int n, double* A, lo
                 double* W) {
   const int nb = h->nb;
   const int m2 = n - k - b;
-  TRY(launch_potrf_diag(st, uplo, A + k + (size_t)k * lda, lda, b, W, nb, h->dstatus, k));
+  TRY(launch_potrf_diag(st, uplo, A + k + (size_t)k * lda, lda, b, m2 > 0 ? W : nullptr, nb, h->dstatus, k));
   if (m2 == 0) return EGPU_OK;
   if (uplo == EGPU_LOWER) {
     double* A21 = A + (k + b) + (size_t)k * lda;

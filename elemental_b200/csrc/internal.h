@@ -118,7 +118,7 @@ int sweep32_prepare(cudaStream_t st, int n, const float* L, long long ldl, const
 int sweep32_solve(cudaStream_t st, int trans, int n, int nrhs, const float* L, long long ldl, double* X,
                   long long ldx, void* ws, int sm_count, DevStatus* status);
 
-// Diagonal-block Cholesky (factor in place + triangular inverse into W).
+// Diagonal-block Cholesky (factor in place + triangular inverse into W unless W is null).
 int launch_potrf_diag(cudaStream_t st, int uplo, double* A, long long lda, int b, double* W, int ldw,
                       DevStatus* status, int col_base, bool store_factor = true);
 // The mixed path's diagonal block: lower Cholesky of the FP32 b x b block at

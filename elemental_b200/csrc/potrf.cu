@@ -49,7 +49,7 @@ __device__ void tri_inverse_smem(double* S, int b, int uplo, int unit) {
 
 // Cholesky of the b x b diagonal block (cholesky::LVar3Unb,
 // lapack-like/Cholesky/LVar3.hpp:19-49, or UVar3Unb, Cholesky/UVar3.hpp:21-50),
-// then the inverse of the factor into W (other triangle zeroed).
+// then the inverse of the factor into W (other triangle zeroed; W may be null).
 template <int UPLO>
 __global__ void __launch_bounds__(kDiagThreads) potrf_diag_kernel(double* A, long long lda, int b, double* W,
                                                                    int ldw, DevStatus* st, int col_base,
@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kDiagThreads) potrf_diag_kernel(double* A, lon
     return;
   }
   if (store_factor) tri_store(S, A, lda, b, UPLO != EGPU_LOWER, false);
+  if (W == nullptr) return;  // the last block: no panel to multiply (the inverse is 12 of 47 us)
   __syncthreads();
   smem_trinv_dmma(S, bp, Xl, T);
   tri_store(S, W, ldw, b, UPLO != EGPU_LOWER, true);  // inv(U) = inv(L)^T

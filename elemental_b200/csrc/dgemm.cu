@@ -272,7 +272,8 @@ static int launch_dgemm_small(cudaStream_t st, bool a_kmajor, bool b_kmajor, int
   cudaError_t e;
   if (alias_a && M <= 16 * 148) e = launch_small_tile<16, 128>(st, a_kmajor, b_kmajor, p);
   else if (alias_a) e = launch_small_tile<32, 128>(st, a_kmajor, b_kmajor, p);
-  else if (alias_b) e = launch_small_tile<128, 16>(st, a_kmajor, b_kmajor, p);
+  else if (alias_b && N <= 16 * 148) e = launch_small_tile<128, 16>(st, a_kmajor, b_kmajor, p);
+  else if (alias_b) e = launch_small_tile<128, 32>(st, a_kmajor, b_kmajor, p);
   else e = launch_small_tile<32, 32>(st, a_kmajor, b_kmajor, p);
   if (e != cudaSuccess) {
     set_last_error(e, "dgemm_small launch", __FILE__, __LINE__);

@@ -250,7 +250,10 @@ int potrf_lookahead(egpu_context* h, int uplo, int n, double* A, long long lda, 
 static const int kRamp[4] = {2, 8, 16, 16};
 
 static int auto_group(int m_left) {
-  return m_left > 12288 ? 16 : m_left > 7168 ? 8 : m_left > 5120 ? 4 : m_left > 3072 ? 2 : 1;
+  // ms at n = 4999 / 6500 / 8192 / 16384: 3.55 / 5.42 / 9.01 / 52.3; with the limits
+  // 12288, 7168, 5120, 3072 3.61 / 5.73 / 9.44 / 52.5; with 14336, 12288, 10240,
+  // 8192 3.56 / 5.53 / 9.00 / 52.7
+  return m_left > 14336 ? 16 : m_left > 10240 ? 8 : m_left > 7168 ? 4 : m_left > 4096 ? 2 : 1;
 }
 
 int potrf_grouped(egpu_context* h, int uplo, int n, double* A, long long lda, double* W, int G) {

@@ -667,12 +667,18 @@ __device__ int lu_factor(T* F, long long ldf, int n, T* P, const BWork& w, doubl
 #pragma unroll
       for (int i = 0; i < NB; ++i) u[i] = (i < b) ? ldv(col + i) : 0.0;
 #pragma unroll
-      for (int i = 1; i < NB; ++i) {
-        if (i < b) {
-          double s = u[i];
+      for (int q = 0; q < NB - 1; ++q) {  // right-looking: L's column q in 16-byte pairs
+        if (q < b) {
+          if (q > 0) u[q] = (double)(T)u[q];
+          const T* lq = P + q * kPLD;
+          if ((q & 1) == 0) u[q + 1] = fma(-ldv(lq + q + 1), u[q], u[q + 1]);
 #pragma unroll
-          for (int q = 0; q < i; ++q) s = fma(-ldv(P + q * kPLD + i), u[q], s);
-          u[i] = (double)(T)s;
+          for (int i = (q + 2) & ~1; i < NB; i += 2) {
+            double l0, l1;
+            ld_pair(lq + i, l0, l1);
+            u[i] = fma(-l0, u[q], u[i]);
+            u[i + 1] = fma(-l1, u[q], u[i + 1]);
+          }
         }
       }
 #pragma unroll

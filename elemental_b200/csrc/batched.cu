@@ -526,7 +526,7 @@ __device__ int lu_panel_smem(T* P, int m, int b, int* s_piv, int* s_mv, int* s_n
 struct BWork {
   double* X;
   double* S;
-  double* col;  // 64 doubles, the leaf factorization's columns
+  double* col;  // 32 doubles, the leaf factorization's column
   double* Y;
   double* BS;
   double* rd;
@@ -998,7 +998,7 @@ __global__ void __launch_bounds__(NT, MINB) batched_kernel(BatchArgs args) {
   constexpr bool kRefined = sizeof(T) == 4;
   constexpr bool kHPD = KIND == 0;
   __shared__ double s_rd[32];
-  __shared__ __align__(16) double s_col[64];
+  __shared__ __align__(16) double s_col[32];
   __shared__ double s_red[3 * kRC * (NT / 32) + 3 * kRC];
   __shared__ int s_piv[32];
   __shared__ int s_mv[2 * 64];

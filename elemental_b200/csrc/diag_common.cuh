@@ -55,65 +55,53 @@ __device__ __forceinline__ int warp_argmax(unsigned long long key, int pos) {
 // ---------------------------------------------------------------------------
 // Building blocks on shared-memory operands (all column-major).
 
-// Pair steps of warp_chol16 from column j0 on, four pairs (NW: the columns after
-// the current pair that can still be needed, 14 or 6).
+// Columns [J0, J0 + 8) of warp_chol16 (NW: the columns after the current one
+// that can still be needed, 15 or 7).
 template <int NW>
-__device__ __forceinline__ void warp_chol16_pairs(double (&z)[16], double& d0, double& b, double& e, int& fail,
-                                                  int j0, bool inv, int i, double* Sd, int lds, double* Xd,
-                                                  double* buf) {
+__device__ __forceinline__ void warp_chol16_cols(double (&z)[16], double& d, int& fail, int j0, bool inv, int i,
+                                                 double* Sd, int lds, double* Xd, double* buf) {
 #pragma unroll 1
-  for (int j = j0; j < j0 + 8; j += 2) {
-    double* cb = buf + (j & 2) * 16;  // two slots: a slow lane may still read the other one
-    if (!inv && i > j + 1) *reinterpret_cast<double2*>(cb + 2 * (i - j - 2)) = make_double2(z[0], z[1]);
-    // the next pair's diagonal block before this pair's update
-    const double auu = __shfl_sync(0xffffffffu, z[2], (j + 2) & 15);
-    const double avu = __shfl_sync(0xffffffffu, z[2], (j + 3) & 15);
-    const double avv = __shfl_sync(0xffffffffu, z[3], (j + 3) & 15);
+  for (int j = j0; j < j0 + 8; ++j) {
+    double* cb = buf + (j & 1) * 16;  // two slots: a slow lane may still read the other one
+    if (!inv && i > j) cb[i - j - 1] = z[0];
+    const double dn = __shfl_sync(0xffffffffu, z[1], (j + 1) & 15);
     __syncwarp();
-    double2 c[NW];  // raw columns j, j + 1 of row j + 2 + k; past the block stale, reaching only columns past it
+    double c[NW + 1];  // a_{j+1+k, j}; entries past the block are stale and only reach columns past it
 #pragma unroll
-    for (int k = 0; k < NW; ++k) c[k] = *reinterpret_cast<const double2*>(cb + 2 * k);
-    const double rs0 = rsqrt(d0);
-    const double l10 = b * rs0;
-    const double d1 = fma(-l10, l10, e);
-    if (fail == 0) fail = d0 <= 0.0 ? j + 1 : d1 <= 0.0 ? j + 2 : 0;
-    const double rs1 = rsqrt(d1);
-    // rows u = j + 2 and v = j + 3 of the factor, for the next diagonal block
-    const double u0 = c[0].x * rs0, u1 = fma(-u0, l10, c[0].y) * rs1;
-    const double v0 = c[1].x * rs0, v1 = fma(-v0, l10, c[1].y) * rs1;
-    d0 = fma(-u1, u1, fma(-u0, u0, auu));
-    b = fma(-v1, u1, fma(-v0, u0, avu));
-    e = fma(-v1, v1, fma(-v0, v0, avv));
-    // this lane's entries, and them times the inverse of the pair's factor
-    const double l0 = z[0] * rs0, l1 = fma(-l0, l10, z[1]) * rs1;
-    const double x1 = l1 * rs1, x0 = fma(-x1, l10, l0) * rs0;
-#pragma unroll
-    for (int k = 0; k < NW; ++k) z[k] = fma(-x1, c[k].y, fma(-x0, c[k].x, z[k + 2]));
-    if (inv) {
-      Xd[j] = l0;
-      Xd[j + 1] = l1;
-    } else {
-      if (i >= j) Sd[j * lds] = l0;
-      if (i >= j + 1) Sd[(j + 1) * lds] = l1;
+    for (int q = 0; q < (NW + 1) / 2; ++q) {
+      const double2 v = *reinterpret_cast<const double2*>(cb + 2 * q);
+      c[2 * q] = v.x;
+      c[2 * q + 1] = v.y;
     }
+    const double rs = rsqrt(d);
+    if (fail == 0 && d <= 0.0) fail = j + 1;
+    c[0] *= rs;
+    d = fma(-c[0], c[0], dn);
+    const double m = z[0] * rs;
+#pragma unroll
+    for (int k = 1; k < NW; ++k) c[k] *= rs;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) z[k] = fma(-m, c[k], z[k + 1]);
+    if (inv) Xd[j] = m;
+    else if (i >= j) Sd[j * lds] = m;
   }
 }
 
 // Cholesky of one 16 x 16 lower block at S[o.., o..] (LVar3Unb,
 // Cholesky/LVar3.hpp:19-49) and the inverse of its factor (into X, 16 x 16, ld
-// ldx, zero above the diagonal) by one warp, in one loop over pairs of columns.
+// ldx, zero above the diagonal) by one warp, in one loop over the columns.
 // Lane i < 16 holds row i of the block, lane 16 + c column c of the identity;
-// registers 0 and 1 are the current pair.  A step is the same for both halves:
-// with the pair's diagonal block [d0; b e] and the raw columns broadcast
-// through shared memory, (l0, l1) = (z_0, z_1) inv(L_p)^T are the finished
-// entries of the factor (of its inverse), and z_k -= (l0, l1) inv(L_p) a_k is
-// the update of A22 (the forward substitution with the factor).  The chain per
-// pair is two reciprocal square roots and the products between them; the
-// broadcast precedes the roots and every lane forms the next pair's diagonal
-// block itself from copies fetched beforehand.  Per block, alone on the SM:
-// 7000 cycles with reciprocal, root and failure test in one chain per column,
-// 5000 with a column's chain of root, product and FMA, 4500 in pairs.
-// buf: 64 doubles of shared memory, 16-byte aligned, of this warp.
+// register 0 is the current column.  Step j, with the raw column a_kj
+// broadcast through shared memory and d = a_jj, is the same for both halves:
+// m = z_0 / sqrt(d) is the finished entry of the factor (of its inverse), and
+// z_k -= m l_kj, l_kj = a_kj / sqrt(d) formed by every lane for itself, is the
+// update of A22 (the forward substitution with the factor).  The chain per
+// column is one reciprocal square root, one multiply and one FMA (55 + 23 + 23
+// cycles here): the broadcast precedes the square root, and the next pivot is
+// formed by every lane from a copy of a_{j+1,j+1} fetched beforehand.
+// Measured per block, alone on the SM: 7000 cycles with the reciprocal, the
+// root and the failure test in the chain one after the other.
+// buf: 32 doubles of shared memory, 16-byte aligned, of this warp.
 // Returns 0 or the 1-based column of a non-positive pivot (warp-uniform).
 __device__ inline int warp_chol16(double* S, int lds, int o, double* X, int ldx, double* buf) {
   const int lane = threadIdx.x & 31, i = lane & 15;
@@ -122,11 +110,10 @@ __device__ inline int warp_chol16(double* S, int lds, int o, double* X, int ldx,
   double z[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) z[k] = inv ? (k == i ? 1.0 : 0.0) : (k <= i ? Sd[k * lds] : 0.0);
-  double d0 = __shfl_sync(0xffffffffu, z[0], 0), b = __shfl_sync(0xffffffffu, z[0], 1),
-         e = __shfl_sync(0xffffffffu, z[1], 1);
+  double d = __shfl_sync(0xffffffffu, z[0], 0);
   int fail = 0;
-  warp_chol16_pairs<14>(z, d0, b, e, fail, 0, inv, i, Sd, lds, X + i * ldx, buf);
-  warp_chol16_pairs<6>(z, d0, b, e, fail, 8, inv, i, Sd, lds, X + i * ldx, buf);
+  warp_chol16_cols<15>(z, d, fail, 0, inv, i, Sd, lds, X + i * ldx, buf);
+  warp_chol16_cols<7>(z, d, fail, 8, inv, i, Sd, lds, X + i * ldx, buf);
   __syncwarp();
   return fail;
 }
@@ -379,7 +366,7 @@ __device__ inline void smem_l21_inplace(double* P, int m2, const double* X11) {
 // pivot (uniform).
 __device__ inline int smem_chol_dmma(double* S, int bp, double* Xl, double* /*T*/) {
   __shared__ int s_fail;
-  __shared__ __align__(16) double s_col[64];
+  __shared__ __align__(16) double s_col[32];
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (warp == 0) {
     const int f = warp_chol16(S, kLDS, 0, Xl, kLeafLD, s_col);

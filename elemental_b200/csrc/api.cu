@@ -462,14 +462,12 @@ static int skinny_pair(egpu_context* h, int n, int nrhs, const double* A, long l
   unsigned char* base = static_cast<unsigned char*>(h->ws) + ws_off;
   double* W1 = reinterpret_cast<double*>(base);
   double* W2 = same ? W1 : reinterpret_cast<double*>(base + wb);
-  int* flags = reinterpret_cast<int*>(base + (same ? 1 : 2) * wb);
+  SweepSeq seq{reinterpret_cast<int*>(base + (same ? 1 : 2) * wb)};
   cudaStream_t st = h->stream;
-  EGPU_CUDA_TRY(cudaMemsetAsync(flags, 0, trsm_skinny_flag_bytes(n, nb), st));
   TRY(launch_trtri_blocks(st, t1.uplo, t1.unit, A, lda, n, nb, W1, nb));
   if (!same) TRY(launch_trtri_blocks(st, t2.uplo, t2.unit, A, lda, n, nb, W2, nb));
-  TRY(launch_trsm_skinny(st, t1.bwd, t1.amode, n, nrhs, A, lda, W1, nb, B, ldb, flags, 1, h->sm_count, h->dstatus));
-  return launch_trsm_skinny(st, t2.bwd, t2.amode, n, nrhs, A, lda, W2, nb, B, ldb, flags, 2, h->sm_count,
-                            h->dstatus);
+  TRY(launch_trsm_skinny(st, t1.bwd, t1.amode, n, nrhs, A, lda, W1, nb, B, ldb, seq, h->sm_count, h->dstatus));
+  return launch_trsm_skinny(st, t2.bwd, t2.amode, n, nrhs, A, lda, W2, nb, B, ldb, seq, h->sm_count, h->dstatus);
 }
 
 // X := inv(T) X with one skinny sweep (workspace from its start).
@@ -480,10 +478,9 @@ static int skinny_single(egpu_context* h, int n, int nrhs, const double* A, long
   TRY(ensure_ws(h, wb + trsm_skinny_flag_bytes(n, nb) + 4096));
   unsigned char* base = static_cast<unsigned char*>(h->ws);
   double* W = reinterpret_cast<double*>(base);
-  int* flags = reinterpret_cast<int*>(base + wb);
-  EGPU_CUDA_TRY(cudaMemsetAsync(flags, 0, trsm_skinny_flag_bytes(n, nb), h->stream));
+  SweepSeq seq{reinterpret_cast<int*>(base + wb)};
   TRY(launch_trtri_blocks(h->stream, t.uplo, t.unit, A, lda, n, nb, W, nb));
-  return launch_trsm_skinny(h->stream, t.bwd, t.amode, n, nrhs, A, lda, W, nb, B, ldb, flags, 1, h->sm_count,
+  return launch_trsm_skinny(h->stream, t.bwd, t.amode, n, nrhs, A, lda, W, nb, B, ldb, seq, h->sm_count,
                             h->dstatus);
 }
 

@@ -64,13 +64,20 @@ int launch_split_tf32_f32(cudaStream_t st, int rows, int cols, const float* X, l
 
 // X := inv(T) X for nrhs <= 64 in one cooperative launch (trsm_skinny.cu:
 // amode/bwd select T from the stored triangle A, Winv the inverted diagonal
-// blocks).  flags: ceil(n/nb) ints that hold values other than `epoch`.
+// blocks).  seq: the arrival counters (trsm_skinny_flag_bytes) of a sequence of
+// sweeps of order n on one stream; the launch keeps its count and zeroes the
+// counters before the first sweep and before one whose CTAs count differently.
 // Y != NULL selects a prescaled A: column-prescaled (X: b in, z out; Y :=
 // inv(T_rr) z_r) or, with row_prescaled, row-prescaled (Y: b in, X := x).
 // Returns EGPU_ERR_UNSUPPORTED when the shape or alignment does not fit.
 size_t trsm_skinny_flag_bytes(int n, int nb);
+struct SweepSeq {
+  int* flags;
+  int epoch = 0;          // sweeps since the counters were zero
+  int groups = 0, strips = 0;  // of those sweeps
+};
 int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, const double* A, long long lda,
-                       const double* Winv, int nb, double* X, long long ldx, int* flags, int epoch, int sm_count,
+                       const double* Winv, int nb, double* X, long long ldx, SweepSeq& seq, int sm_count,
                        DevStatus* status, double* Y = nullptr, bool row_prescaled = false);
 
 // C += alpha A B for N <= 64 (split-K DMMA, FP64 atomics into C); A, B

@@ -237,8 +237,7 @@ static MixedLayout mixed_layout(int n, int nrhs, int nb) {
 // Y := W z) and the row-prescaled backward sweep over M2^T (Y in, X out).
 // Otherwise Lf holds L and the blocked multiply-by-inverse form runs.
 struct SweepFlags {
-  int* flags;
-  int epoch;
+  SweepSeq seq;
   bool prescaled;
   double* Y;
   const float* Lf32;  // non-null: the FP32 super-block sweeps over this factor
@@ -249,10 +248,10 @@ static int mixed_solve(egpu_context* h, int n, int nrhs, const double* Lf, long 
                        double* X, SweepFlags& fl) {
   if (fl.Lf32) return sweep32_solve(h->stream, 2, n, nrhs, fl.Lf32, fl.ldf, X, lds, fl.sw, h->sm_count, h->dstatus);
   if (fl.prescaled) {
-    TRY(launch_trsm_skinny(h->stream, 0, 0, n, nrhs, Lf, lds, Winv, h->nb, X, lds, fl.flags, ++fl.epoch,
-                           h->sm_count, h->dstatus, fl.Y));
-    return launch_trsm_skinny(h->stream, 1, 1, n, nrhs, Lf, lds, Winv, h->nb, X, lds, fl.flags, ++fl.epoch,
-                              h->sm_count, h->dstatus, fl.Y, true);
+    TRY(launch_trsm_skinny(h->stream, 0, 0, n, nrhs, Lf, lds, Winv, h->nb, X, lds, fl.seq, h->sm_count,
+                           h->dstatus, fl.Y));
+    return launch_trsm_skinny(h->stream, 1, 1, n, nrhs, Lf, lds, Winv, h->nb, X, lds, fl.seq, h->sm_count,
+                              h->dstatus, fl.Y, true);
   }
   TRY(trsm_blocked(h->stream, EGPU_LEFT, EGPU_LOWER, 0, n, nrhs, Lf, lds, Winv, h->nb, X, lds, h->dstatus));
   return trsm_blocked(h->stream, EGPU_LEFT, EGPU_LOWER, 1, n, nrhs, Lf, lds, Winv, h->nb, X, lds, h->dstatus);
@@ -501,14 +500,13 @@ int dposv_mixed_core_impl(egpu_context* h, int uplo, int n, int nrhs, const doub
   double* norms = reinterpret_cast<double*>(ws + L.norms);
   // prescaled sweeps where the one-launch sweep kernel takes the shape
   const bool prescale = nrhs <= 64 && nb >= 8 && nb <= 128 && nb % 2 == 0;
-  SweepFlags fl{reinterpret_cast<int*>(ws + L.flags), 0, prescale, reinterpret_cast<double*>(ws + L.yt), nullptr,
+  SweepFlags fl{{reinterpret_cast<int*>(ws + L.flags)}, prescale, reinterpret_cast<double*>(ws + L.yt), nullptr,
                 0, ws + L.sw};
   // the FP32 super-block sweeps take the corrections when the panels are 128
   // wide and the FP32 factor is TMA-addressable; the FP64 copy of L (and its
   // prescaled M2 form) is then only built if GMRES-IR needs it
   const bool use32 = nb == 128 && nrhs <= 32 && L.ldf % 4 == 0;
   bool have_lf = false;  // Lf holds the FP64 copy (prescaled when `prescale`)
-  EGPU_CUDA_TRY(cudaMemsetAsync(fl.flags, 0, trsm_skinny_flag_bytes(n, nb), st));
   const long long lds = L.lds, ldf = L.ldf;
   // The factorization: the fast form computes every panel's L21 on the
   // tensor cores (TF32 x 3); `accurate` keeps L21 in FP64 (DMMA), a second

@@ -293,7 +293,7 @@ int dgesv_mixed_core(egpu_context* h, int n, int nrhs, const double* A, long lon
   float *Lh = reinterpret_cast<float*>(ws + L.lh), *Ll = reinterpret_cast<float*>(ws + L.ll);
   double* WinvL = reinterpret_cast<double*>(ws + L.winvl);
   double* WinvU = reinterpret_cast<double*>(ws + L.winvu);
-  int* flags = reinterpret_cast<int*>(ws + L.flags);
+  SweepSeq seq{reinterpret_cast<int*>(ws + L.flags)};  // of the solves and of the condition estimate's one column
   int* perm = reinterpret_cast<int*>(ws + L.perm);
   double* Xw = reinterpret_cast<double*>(ws + L.xw);
   double* R = reinterpret_cast<double*>(ws + L.r);
@@ -398,7 +398,6 @@ int dgesv_mixed_core(egpu_context* h, int n, int nrhs, const double* A, long lon
   TRY(launch_compose_perm(st, 0, n, piv, n, permF));
   TRY(launch_compose_perm(st, 1, n, piv, n, permI));
   bool have64 = false;
-  int epoch = 0;
   auto materialize64 = [&]() -> int {  // FP64 factors and their block inverses
     if (have64) return EGPU_OK;
     widen_kernel<<<dim3((n + 255) / 256, std::min(n, 65535)), 256, 0, st>>>(n, n, Af, ldf, LU, lds);
@@ -406,7 +405,6 @@ int dgesv_mixed_core(egpu_context* h, int n, int nrhs, const double* A, long lon
     EGPU_CUDA_TRY(cudaGetLastError());
     if (!use32) TRY(launch_trtri_blocks(st, EGPU_LOWER, 1, LU, lds, n, nb, WinvL, nb));
     TRY(launch_trtri_blocks(st, EGPU_UPPER, 0, LU, lds, n, nb, WinvU, nb));
-    EGPU_CUDA_TRY(cudaMemsetAsync(flags, 0, trsm_skinny_flag_bytes(n, nb), st));
     have64 = true;
     return EGPU_OK;
   };
@@ -414,15 +412,11 @@ int dgesv_mixed_core(egpu_context* h, int n, int nrhs, const double* A, long lon
     TRY(materialize64());
     if (!trans) {
       TRY(launch_permute_rows(st, n, ncols, permF, V, lds, ptmp));
-      TRY(launch_trsm_skinny(st, 0, 0, n, ncols, LU, lds, WinvL, nb, V, lds, flags, ++epoch, h->sm_count,
-                             h->dstatus));
-      return launch_trsm_skinny(st, 1, 0, n, ncols, LU, lds, WinvU, nb, V, lds, flags, ++epoch, h->sm_count,
-                                h->dstatus);
+      TRY(launch_trsm_skinny(st, 0, 0, n, ncols, LU, lds, WinvL, nb, V, lds, seq, h->sm_count, h->dstatus));
+      return launch_trsm_skinny(st, 1, 0, n, ncols, LU, lds, WinvU, nb, V, lds, seq, h->sm_count, h->dstatus);
     }
-    TRY(launch_trsm_skinny(st, 0, 1, n, ncols, LU, lds, WinvU, nb, V, lds, flags, ++epoch, h->sm_count,
-                           h->dstatus));
-    TRY(launch_trsm_skinny(st, 1, 1, n, ncols, LU, lds, WinvL, nb, V, lds, flags, ++epoch, h->sm_count,
-                           h->dstatus));
+    TRY(launch_trsm_skinny(st, 0, 1, n, ncols, LU, lds, WinvU, nb, V, lds, seq, h->sm_count, h->dstatus));
+    TRY(launch_trsm_skinny(st, 1, 1, n, ncols, LU, lds, WinvL, nb, V, lds, seq, h->sm_count, h->dstatus));
     return launch_permute_rows(st, n, ncols, permI, V, lds, ptmp);
   };
   auto lu_solve = [&](double* V, int ncols, int trans) -> int {

@@ -411,11 +411,12 @@ size_t trsm_skinny_flag_bytes(int n, int nb) {
   return sizeof(int) * (size_t)((n + nb - 1) / nb) * kTsMaxGroups + 256;
 }
 
-// flags: device array (trsm_skinny_flag_bytes) of arrival counters, zero before the first
-// sweep of a sequence; sweep number `epoch` (1, 2, ...) of the sequence
-// waits for counters to reach strips x epoch.
+// Sweep number `epoch` (1, 2, ...) since the counters were zero waits for them
+// to reach strips x epoch.  Each group of right-hand sides has its own
+// counters, so all those sweeps must have had the same groups and strips: a
+// sweep with others (another number of right-hand sides) starts from zero.
 int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, const double* L, long long lda,
-                       const double* Winv, int nb, double* X, long long ldx, int* flags, int epoch, int sm_count,
+                       const double* Winv, int nb, double* X, long long ldx, SweepSeq& seq, int sm_count,
                        DevStatus* status, double* Y, bool row_prescaled) {
   if (n <= 0 || nrhs <= 0) return EGPU_OK;
   if (nrhs > kTsMaxRhs || nb > 128 || nb < 8 || nb % 2 != 0 || ldx % 2 != 0 || lda % 2 != 0 ||
@@ -431,7 +432,7 @@ int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, con
   // catch up with all the products of its block row)
   p.strips = (p.mode != 0 && nb >= 32 && p.nblk <= sm_count) ? 2 : 1;
   p.hs = p.strips == 1 ? nb : ((nb + 1) / 2 + 15) / 16 * 16;
-  p.flags = flags; p.epoch = epoch; p.status = status;
+  p.flags = seq.flags; p.status = status;
   // the A pieces: TMA boxes over the stored n x n matrix and over the Winv
   // slots (nb rows x nblk*nb columns), the same box for both
   const uint32_t bi = amode == 0 ? (uint32_t)(p.hs + 4) : (uint32_t)kTsCT;
@@ -472,6 +473,17 @@ int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, con
     }
     attr[ai] = true;
   }
+  if (seq.epoch == 0 || seq.groups != p.groups || seq.strips != p.strips) {
+    const cudaError_t ez = cudaMemsetAsync(seq.flags, 0, trsm_skinny_flag_bytes(n, nb), st);
+    if (ez != cudaSuccess) {
+      set_last_error(ez, "trsm_skinny counters", __FILE__, __LINE__);
+      return EGPU_ERR_CUDA;
+    }
+    seq.epoch = 0;
+    seq.groups = p.groups;
+    seq.strips = p.strips;
+  }
+  p.epoch = ++seq.epoch;
   const int grid = p.groups * p.gsz;
   TraceMark tm(st, kTraceSolve, (double)n * n * p.nrhs, 4.0 * (double)n * n + 16.0 * n * p.nrhs);
   cudaLaunchConfig_t cfg = {};

@@ -263,6 +263,26 @@ def test_gaussian_elimination_mixed_ill_conditioned(handle, kind, kappa, mode, p
         assert k1 / 10 <= est <= k1 * 10, (est, k1)
 
 
+# more than 32 right-hand sides: the FP64 sweeps, in groups of 8; the condition
+# estimate's solves of one column come between theirs
+@pytest.mark.parametrize("nrhs", [33, 64])
+@pytest.mark.parametrize("policy,kappa", [(1, 1e4), (1, 3e7), (0, 3e7)])
+def test_gaussian_elimination_mixed_estimate_between_wide_solves(handle, policy, kappa, nrhs):
+    n = 600
+    A, B = inputs.general_spectrum(n, kappa, 79), inputs.normal(n, nrhs, 80)
+    handle.set_mixed_policy(policy)
+    try:
+        X, it, be = handle.gaussian_elimination_mixed(eg.colmajor_cuda(A), eg.colmajor_cuda(B))
+        est = handle.mixed_condition_estimate()
+    finally:
+        handle.set_mixed_policy(0)
+    assert it >= 1
+    assert be <= 1e-14 and _berr(A, X.cpu().numpy(), B) <= 1e-14
+    if policy == 1:
+        k1 = np.linalg.cond(A, 1)
+        assert k1 / 10 <= est <= k1 * 10, (est, k1)
+
+
 def test_gaussian_elimination_mixed_singular(handle):
     n = 300
     A = inputs.uniform(n, n, 75)

@@ -133,6 +133,7 @@ def _declare(L):
         "egpu_batch_plan_info": ([P, P, P], I),
         "egpu_batch_plan_autotune": ([P, P, I, P, P], I),
         "egpu_batch_plan_set_grid": ([P, I], I),
+        "egpu_batch_plan_set_shape": ([P, I, I], I),
         "egpu_batch_plan_destroy": ([P], I),
         "egpu_server_create": ([I, ctypes.c_size_t, I, I, P], I),
         "egpu_server_set_tolerance": ([P, D], I),
@@ -416,6 +417,10 @@ class BatchPlan:
 
     def set_grid(self, grid):
         _check(lib().egpu_batch_plan_set_grid(self._p, grid))
+
+    def set_shape(self, panel, threads):
+        """One launch of this shape (as shape() reports it) over all systems."""
+        _check(lib().egpu_batch_plan_set_shape(self._p, panel, threads))
 
     def iters(self, stream=None):
         """Refinement corrections per system of the last run (-1: the system

@@ -1160,6 +1160,12 @@ int egpu_batch_plan_set_grid(egpu_batch_plan plan, int grid) {
   return EGPU_OK;
 }
 
+int egpu_batch_plan_set_shape(egpu_batch_plan plan, int panel, int threads) {
+  if (!plan) return EGPU_ERR_ARG;
+  Enter g(plan->h);
+  return egpu::batch_plan_set_shape(plan->p, panel, threads);
+}
+
 int egpu_batch_plan_destroy(egpu_batch_plan plan) {
   if (!plan) return EGPU_OK;
   {

@@ -60,8 +60,14 @@ constexpr int kIRMax = 10;                     // refinement corrections before 
 constexpr double kIRTol = 1e-14;               // backward error the refined plans reach
 constexpr int kScrDoubles = kBmaxN * 32 + kBmaxN / 2;  // per-CTA scratch: inverses + interchanges
 
+// Leading dimension of a diagonal block in shared memory: the leaves are 16
+// wide, so an 8-wide block (the refined plans' FP64 fallback) takes 16 rows and
+// columns too.
+constexpr int diag_w(int NB) { return NB < 16 ? 16 : NB; }
+constexpr int diag_ld(int NB) { return diag_w(NB) + 4; }
+
 // Shared-memory layout (bytes) for storage type T and panel width NB: the
-// panel P, the diagonal-block inverse / solve staging X (NB x (NB + 4)), the
+// panel P, the diagonal-block inverse / solve staging X (diag_w(NB) x diag_ld(NB)), the
 // diagonal block in FP64 while it is factored S (the same size), the
 // left-looking dots Y (NB x kRC) and, for refined plans whose panel is
 // smaller than two right-hand-side chunks, the solution chunk BS.  The
@@ -70,16 +76,16 @@ constexpr int kScrDoubles = kBmaxN * 32 + kBmaxN / 2;  // per-CTA scratch: inver
 constexpr size_t kChunkBytes = (size_t)kRC * kBmaxN * 8;
 template <typename T, int NB>
 struct BL {
-  static constexpr int kXLD = NB + 4;
+  static constexpr int kXLD = diag_ld(NB);
   static constexpr size_t kPBytes = (size_t)NB * kPLD * sizeof(T);
   static constexpr bool kOwnBS = sizeof(T) == 4 && kPBytes < 2 * kChunkBytes;
   static constexpr size_t kOffX = (kPBytes + 15) & ~size_t(15);
-  static constexpr size_t kOffS = kOffX + (size_t)NB * kXLD * 8;
-  static constexpr size_t kOffY = kOffS + (size_t)NB * kXLD * 8;
+  static constexpr size_t kOffS = kOffX + (size_t)diag_w(NB) * kXLD * 8;
+  static constexpr size_t kOffY = kOffS + (size_t)diag_w(NB) * kXLD * 8;
   static constexpr size_t kOffB = kOffY + (size_t)NB * kRC * 8;
   static constexpr size_t kBytes = kOffB + (kOwnBS ? kChunkBytes : 0);
   static_assert(kPBytes >= kChunkBytes, "the solves' chunk aliases the panel");
-  static_assert((size_t)NB * kXLD * 8 >= 2 * 8 * (2 + NB / 2) * 16, "the panel's candidates (8 warps) fit S");
+  static_assert((size_t)diag_w(NB) * kXLD * 8 >= 2 * 8 * (2 + NB / 2) * 16, "the panel's candidates (8 warps) fit S");
 };
 
 struct BatchArgs {
@@ -287,20 +293,21 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
 }
 
 // ------------------------------------------------ diagonal-block kernels --
-// Lower Cholesky of the b x b top of the panel (b <= NB, NB 16 or 32) and the
-// inverse of its factor (into X, ld NB + 4, lower part) by one warp: the block
-// in FP64 in S (ld NB + 4, padded with identity), factored and inverted in
+// Lower Cholesky of the b x b top of the panel (b <= NB, NB 8, 16 or 32) and
+// the inverse of its factor (into X, lower part) by one warp: the block in FP64
+// in S (both diag_w(NB) wide, ld diag_ld(NB), padded with identity), factored and inverted in
 // 16-column leaves with the 16 x 16 products between them on DMMA.  The factor
 // goes back to P rounded to T.  Bound by the leaves' chains: 32 columns took
 // 23 us as one unrolled register loop (its code alone 250 KB), 6 us this way.
 // Returns 0 or the 1-based column of a non-positive pivot (warp-uniform).
 template <typename T, int NB>
 __device__ int diag_chol_warp(T* P, int b, double* S, double* X, double* col) {
-  constexpr int LD = NB + 4;
+  static_assert(NB == 8 || NB == 16 || NB == 32, "one leaf or two");
+  constexpr int LD = diag_ld(NB);
   const int lane = threadIdx.x & 31;
-  if (lane < NB) {
+  if (lane < diag_w(NB)) {
 #pragma unroll 8
-    for (int c = 0; c < NB; ++c)
+    for (int c = 0; c < diag_w(NB); ++c)
       if (c <= lane) S[lane + c * LD] = lane < b ? ldv(P + c * kPLD + lane) : (lane == c ? 1.0 : 0.0);
   }
   __syncwarp();
@@ -323,7 +330,7 @@ __device__ int diag_chol_warp(T* P, int b, double* S, double* X, double* col) {
   if (f) return f;
   if (lane < b) {
 #pragma unroll 8
-    for (int c = 0; c < NB; ++c)
+    for (int c = 0; c < NB; ++c)  // c <= lane < b <= NB
       if (c <= lane) stv(P + c * kPLD + lane, S[lane + c * LD]);
   }
   __syncwarp();
@@ -522,7 +529,7 @@ __device__ int lu_panel_smem(T* P, int m, int b, int* s_piv, int* s_mv, int* s_n
 
 // ------------------------------------------------------------ factorizations --
 // Shared-memory work areas of one CTA (pointers into the dynamic block plus
-// the static scalars); X and S are NB x (NB + 4), Y is NB x kRC doubles.
+// the static scalars); X and S are diag_w(NB) x diag_ld(NB), Y is NB x kRC doubles.
 struct BWork {
   double* X;
   double* S;
@@ -542,7 +549,7 @@ struct BWork {
 // blocks, ld NB).  Returns 0 or the 1-based column of a non-positive pivot.
 template <typename T, int NB, int NT>
 __device__ int chol_factor(T* F, long long ldf, int n, T* P, const BWork& w, double* Xg) {
-  constexpr int kXLD = NB + 4;
+  constexpr int kXLD = diag_ld(NB);
   const int tid = threadIdx.x, warp = tid >> 5;
   const bool cvec = (reinterpret_cast<uintptr_t>(F) % (2 * sizeof(T)) == 0) && (ldf % 2 == 0);
   for (int k0 = 0; k0 < n; k0 += NB) {
@@ -610,7 +617,7 @@ __device__ int chol_factor(T* F, long long ldf, int n, T* P, const BWork& w, dou
 // column of a zero pivot.
 template <typename T, int NB, int NT>
 __device__ int lu_factor(T* F, long long ldf, int n, T* P, const BWork& w, double* Xg, int* piv) {
-  constexpr int kXLD = NB + 4;
+  constexpr int kXLD = diag_ld(NB);
   constexpr int NW = NT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool cvec = (reinterpret_cast<uintptr_t>(F) % (2 * sizeof(T)) == 0) && (ldf % 2 == 0);
@@ -1255,16 +1262,20 @@ struct BatchPlan {
   int cvar[kMaxClass] = {0, 0, 0}, cgrid[kMaxClass] = {0, 0, 0}, cnmax[kMaxClass] = {kBmaxN, 0, 0};
 };
 
-static int plan_default_shape(BatchPlan* p) {
+static int plan_single_shape(BatchPlan* p, int var) {
+  int per_sm = 1;
+  BTRY(variant_prepare(kVariants[p->precision][var], p->kind, &per_sm));
   p->nclass = 1;
   p->cbeg[0] = 0;
   p->cend[0] = p->count;
-  p->cvar[0] = default_variant(p->kind, p->precision, p->count > 0 ? p->items[0].n : 0);
+  p->cvar[0] = var;
   p->cnmax[0] = kBmaxN;
-  int per_sm = 1;
-  BTRY(variant_prepare(kVariants[p->precision][p->cvar[0]], p->kind, &per_sm));
   p->cgrid[0] = per_sm * p->sm_count;
   return EGPU_OK;
+}
+
+static int plan_default_shape(BatchPlan* p) {
+  return plan_single_shape(p, default_variant(p->kind, p->precision, p->count > 0 ? p->items[0].n : 0));
 }
 
 int batch_plan_create(int device, int sm_count, int kind, int precision, int count, const int* n, const int* nrhs,
@@ -1528,6 +1539,15 @@ int batch_plan_autotune(BatchPlan* p, cudaStream_t st, int reps, double* best_ms
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   return rc;
+}
+
+// One launch of the given shape over all systems (a candidate of the autotuner).
+int batch_plan_set_shape(BatchPlan* p, int panel, int threads) {
+  for (int v = 0; v < kNumVariants; ++v) {
+    if (kVariants[p->precision][v].nb != panel || kVariants[p->precision][v].nt != threads) continue;
+    return plan_single_shape(p, v);
+  }
+  return EGPU_ERR_ARG;
 }
 
 void batch_plan_set_grid(BatchPlan* p, int grid) {

@@ -183,6 +183,7 @@ int batch_plan_info(BatchPlan* p, cudaStream_t st, int* info_host);
 int batch_plan_iters(BatchPlan* p, cudaStream_t st, int* iters_host);
 int batch_plan_shape(BatchPlan* p, int* nclass, int* class_nmax, int* panel, int* threads, int* grid);
 int batch_plan_autotune(BatchPlan* p, cudaStream_t st, int reps, double* best_ms, int* best_grid);
+int batch_plan_set_shape(BatchPlan* p, int panel, int threads);
 void batch_plan_set_grid(BatchPlan* p, int grid);
 void batch_plan_destroy(BatchPlan* p);
 // kind 0: HPDSolve (lower Cholesky + solve); kind 1: GaussianElimination (LU + solve)

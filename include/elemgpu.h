@@ -191,6 +191,10 @@ EGPU_API int egpu_batch_plan_info(egpu_batch_plan plan, void* stream, int* info)
 EGPU_API int egpu_batch_plan_autotune(egpu_batch_plan plan, void* stream, int reps, double* best_ms,
                                       int* best_grid);
 EGPU_API int egpu_batch_plan_set_grid(egpu_batch_plan plan, int grid);
+/* One launch over all systems with this panel width and CTA size (a choice
+ * that egpu_batch_plan_shape reported before); EGPU_ERR_ARG when the plan's
+ * precision has no such shape. */
+EGPU_API int egpu_batch_plan_set_shape(egpu_batch_plan plan, int panel, int threads);
 /* As egpu_batch_plan_create with a precision: 0 = FP64 (as above); 1 = each
  * system is converted once into an FP32 working copy (plan-owned), factored
  * there (FP64 register arithmetic, values stored in FP32), and its solution

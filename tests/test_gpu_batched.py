@@ -186,6 +186,35 @@ def test_refined_plan_falls_back_to_fp64(handle):
     plan.close()
 
 
+# every launch shape: the FP64 fallback's panel is half the shape's (8, 16), its
+# last block whole (160), ragged (163) or the only one (5)
+@pytest.mark.parametrize("panel,threads", [(32, 256), (16, 256), (32, 128)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_refined_plan_falls_back_in_every_shape(handle, kind, panel, threads):
+    if kind == 0:
+        ill = [inputs.spd_spectrum(n, 1e12, 2 + n) for n in (5, 160, 163)]
+    else:
+        ill = [inputs.general_spectrum(n, 1e12, 2 + n) for n in (5, 160, 163)]
+    stop = inputs.spd_ggt(200, 1)
+    if kind == 0:
+        stop[70, 70] = -3.0
+    else:
+        stop[:, 70] = 0.0
+    mats = [np.asfortranarray(a) for a in ill + [stop]]
+    Bs = [inputs.normal(m.shape[0], 3, 10 + i) for i, m in enumerate(mats)]
+    dA = [eg.colmajor_cuda(m) for m in mats]
+    dB = [eg.colmajor_cuda(b) for b in Bs]
+    plan = eg.BatchPlan(handle, kind, dA, dB, precision=1)
+    plan.set_shape(panel, threads)
+    assert [(s["panel"], s["threads"]) for s in plan.shape()] == [(panel, threads)]
+    plan.run()
+    assert plan.info() == [0, 0, 0, 71]
+    assert plan.iters()[1:] == [-1] * 3
+    for i in range(3):
+        assert _berr(mats[i], dB[i].cpu().numpy(), Bs[i]) <= 1e-14, i
+    plan.close()
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 def test_autotune_restores_inputs_and_reports_shapes(handle, precision):
     """The tile-shape autotuner leaves every input as it found it, reports a

@@ -443,7 +443,7 @@ int trsm_core(egpu_context* h, int side, int uplo, int trans, int unit, int m, i
 
 // Can the one-launch skinny sweep (trsm_skinny.cu) take this right-hand side?
 static bool skinny_ok(egpu_context* h, int nrhs, const double* A, long long lda, const double* B, long long ldb) {
-  return nrhs >= 1 && nrhs <= 64 && h->nb <= 128 && h->nb % 2 == 0 && ldb % 2 == 0 && lda % 2 == 0 &&
+  return nrhs >= 1 && nrhs <= 64 && h->nb >= 8 && h->nb <= 128 && h->nb % 2 == 0 && ldb % 2 == 0 && lda % 2 == 0 &&
          reinterpret_cast<uintptr_t>(B) % 16 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
 }
 

@@ -167,6 +167,27 @@ def test_gaussian_elimination_routes(handle, n, nrhs):
     assert solve_bwd(A, host(dB), B) <= 4
 
 
+# block sizes that the one-launch sweeps do not take, and the smallest that they do
+@pytest.mark.parametrize("nb", [2, 6, 8])
+@pytest.mark.parametrize("n,nrhs", [(20, 3), (50, 64)])
+def test_solves_with_small_block_sizes(handle, n, nrhs, nb):
+    import torch
+    A, S, B = inputs.uniform(n, n, 22), inputs.spd_ggt(n, 23), inputs.normal(n, nrhs, 24)
+    old = handle.blocksize()
+    handle.set_blocksize(nb)
+    try:
+        dX, dY, dZ, dF, p = cuda(B), cuda(B), cuda(B), cuda(A), torch.zeros(n, dtype=torch.int32, device="cuda")
+        handle.gaussian_elimination(cuda(A), dX)
+        handle.hpd_solve(cuda(S), dY)
+        handle.lu(dF, p)
+        handle.lu_solve_after(dF, p, dZ)
+    finally:
+        handle.set_blocksize(old)
+    assert solve_bwd(A, host(dX), B) <= 4
+    assert solve_bwd(S, host(dY), B) <= 4
+    assert solve_bwd(A, host(dZ), B) <= 4
+
+
 # the shapes change with the largest order; block edges at multiples of 16 and 32
 @pytest.mark.parametrize("sizes", [(1, 2, 15, 16, 17, 31, 32, 33, 47, 64, 255, 256), (48, 257, 300, 511, 512)])
 def test_batched_block_edges(handle, sizes):

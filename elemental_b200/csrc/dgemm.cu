@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(const SmallParams p) {
   extern __shared__ __align__(16) double ss[];
   constexpr int TILES = (TM / 16) * (TN / 8), PER = TILES / 8;  // 16 x 8 DMMA tiles per warp
   static_assert(TILES % 8 == 0, "eight warps");
-  if (p.status != nullptr && p.status->code != 0) return;
+  __shared__ int s_go;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * TM, col0 = blockIdx.y * TN;
@@ -155,8 +155,12 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(const SmallParams p) {
       cc[j][r] = v ? p.C[m + (long long)n * p.ldc] : 0.0;
       acc[j][r] = 0.0;
     }
+  // an earlier step failed: the CTA takes one thread's reading (another stream
+  // may set the status meanwhile), made while the copies are in flight
+  if (threadIdx.x == 0) s_go = p.status == nullptr || ((const volatile DevStatus*)p.status)->code == 0;
   cp_async_wait_all();
   __syncthreads();
+  if (!s_go) return;
   const int as = AK ? 1 : small_ld(TM), am = AK ? KP + 4 : 1;  // k and row strides
   const int bs = BK ? 1 : small_ld(TN), bn = BK ? KP + 4 : 1;
   const double* pa = sA + (16 * rt + g) * am + t * as;

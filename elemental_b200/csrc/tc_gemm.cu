@@ -145,7 +145,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (p.status != nullptr && ((volatile DevStatus*)p.status)->code != 0) return;  // uniform
+  // an earlier step failed: the CTA takes one thread's reading (the panel
+  // stream may set the status meanwhile)
+  __shared__ int s_go;
+  if (tid == 0) s_go = p.status == nullptr || ((volatile DevStatus*)p.status)->code == 0;
+  __syncthreads();
+  if (!s_go) return;
   const int KT = (p.K + kTcBK - 1) / kTcBK;
   // a contiguous run of `per_cta` tiles per CTA: CTAs retire every few tiles,
   // so kernels of a higher-priority stream (the look-ahead panel chain) get

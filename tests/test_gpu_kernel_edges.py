@@ -167,6 +167,22 @@ def test_gaussian_elimination_routes(handle, n, nrhs):
     assert solve_bwd(A, host(dB), B) <= 4
 
 
+def tiny_block(n, rows, cols):
+    """I + 2^-55 in a block: a row's products with x = 1 vanish against 1 one by
+    one (half an ulp below 1 is 2^-54), their sum of w 2^-55 does not."""
+    A = np.eye(n)
+    A[rows, cols] = 2.0 ** -55
+    return np.asfortranarray(A)
+
+
+@pytest.mark.parametrize("nrhs", [1, 16, 64])
+def test_last_solve_sums_a_block_before_it_meets_b(handle, nrhs):
+    A = tiny_block(256, slice(0, 128), slice(128, 256))
+    dB = cuda(np.ones((256, nrhs), order="F"))
+    handle.gaussian_elimination(cuda(A), dB)
+    assert (host(dB)[:128] == 1.0 - 2.0 ** -48).all() and (host(dB)[128:] == 1.0).all()
+
+
 # block sizes that the one-launch sweeps do not take, and the smallest that they do
 @pytest.mark.parametrize("nb", [2, 6, 8])
 @pytest.mark.parametrize("n,nrhs", [(20, 3), (50, 64)])

@@ -183,6 +183,19 @@ def test_last_solve_sums_a_block_before_it_meets_b(handle, nrhs):
     assert (host(dB)[:128] == 1.0 - 2.0 ** -48).all() and (host(dB)[128:] == 1.0).all()
 
 
+# products of 32 columns (16-column panels: two sums) right of or left of the diagonal
+@pytest.mark.parametrize("n", [64, 320])
+@pytest.mark.parametrize("lower", [False, True])
+def test_batched_solve_sums_a_block_before_it_meets_b(handle, lower, n):
+    first, last = slice(0, 32), slice(n - 32, n)
+    A = tiny_block(n, last, first) if lower else tiny_block(n, first, last)
+    dB = [cuda(np.ones((n, 3), order="F"))]
+    assert handle.gaussian_elimination_batched([cuda(A)], dB) == [0]
+    want = np.ones((n, 3))
+    want[last if lower else first] = 1.0 - 2.0 ** -50
+    assert np.array_equal(host(dB[0]), want)
+
+
 # block sizes that the one-launch sweeps do not take, and the smallest that they do
 @pytest.mark.parametrize("nb", [2, 6, 8])
 @pytest.mark.parametrize("n,nrhs", [(20, 3), (50, 64)])

@@ -58,8 +58,8 @@ __device__ __forceinline__ int warp_argmax(unsigned long long key, int pos) {
 // Columns [J0, J0 + 8) of warp_chol16 (NW: the columns after the current one
 // that can still be needed, 15 or 7).
 template <int NW>
-__device__ __forceinline__ void warp_chol16_cols(double (&z)[16], double& d, int& fail, int j0, bool inv, int i,
-                                                 double* Sd, int lds, double* Xd, double* buf) {
+__device__ __forceinline__ void warp_chol16_cols(double (&z)[16], double& d, double& mine, int& fail, int j0, bool inv,
+                                                 int i, double* Sd, int lds, double* Xd, double* buf) {
 #pragma unroll 1
   for (int j = j0; j < j0 + 8; ++j) {
     double* cb = buf + (j & 1) * 16;  // two slots: a slow lane may still read the other one
@@ -75,6 +75,7 @@ __device__ __forceinline__ void warp_chol16_cols(double (&z)[16], double& d, int
     }
     const double rs = rsqrt(d);
     if (fail == 0 && d <= 0.0) fail = j + 1;
+    if (i == j) mine = d;
     c[0] *= rs;
     d = fma(-c[0], c[0], dn);
     const double m = z[0] * rs;
@@ -83,7 +84,7 @@ __device__ __forceinline__ void warp_chol16_cols(double (&z)[16], double& d, int
 #pragma unroll
     for (int k = 0; k < NW; ++k) z[k] = fma(-m, c[k], z[k + 1]);
     if (inv) Xd[j] = m;
-    else if (i >= j) Sd[j * lds] = m;
+    else if (i > j) Sd[j * lds] = m;
   }
 }
 
@@ -98,7 +99,10 @@ __device__ __forceinline__ void warp_chol16_cols(double (&z)[16], double& d, int
 // update of A22 (the forward substitution with the factor).  The chain per
 // column is one reciprocal square root, one multiply and one FMA (55 + 23 + 23
 // cycles here): the broadcast precedes the square root, and the next pivot is
-// formed by every lane from a copy of a_{j+1,j+1} fetched beforehand.
+// formed by every lane from a copy of a_{j+1,j+1} fetched beforehand.  The
+// diagonal itself is each lane's root of its own pivot, all 16 side by side at
+// the end: d times the reciprocal root is up to an ulp off, and NaN for an
+// infinite pivot (whose column is 0 and whose row of the inverse is 0).
 // Measured per block, alone on the SM: 7000 cycles with the reciprocal, the
 // root and the failure test in the chain one after the other.
 // buf: 32 doubles of shared memory, 16-byte aligned, of this warp.
@@ -110,10 +114,11 @@ __device__ inline int warp_chol16(double* S, int lds, int o, double* X, int ldx,
   double z[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) z[k] = inv ? (k == i ? 1.0 : 0.0) : (k <= i ? Sd[k * lds] : 0.0);
-  double d = __shfl_sync(0xffffffffu, z[0], 0);
+  double d = __shfl_sync(0xffffffffu, z[0], 0), mine = 1.0;
   int fail = 0;
-  warp_chol16_cols<15>(z, d, fail, 0, inv, i, Sd, lds, X + i * ldx, buf);
-  warp_chol16_cols<7>(z, d, fail, 8, inv, i, Sd, lds, X + i * ldx, buf);
+  warp_chol16_cols<15>(z, d, mine, fail, 0, inv, i, Sd, lds, X + i * ldx, buf);
+  warp_chol16_cols<7>(z, d, mine, fail, 8, inv, i, Sd, lds, X + i * ldx, buf);
+  if (!inv) Sd[i * lds] = sqrt(mine);
   __syncwarp();
   return fail;
 }

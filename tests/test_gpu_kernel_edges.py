@@ -183,6 +183,34 @@ def test_last_solve_sums_a_block_before_it_meets_b(handle, nrhs):
     assert (host(dB)[:128] == 1.0 - 2.0 ** -48).all() and (host(dB)[128:] == 1.0).all()
 
 
+@pytest.mark.parametrize("n", [7, 100, 257])
+def test_cholesky_of_a_diagonal_matrix_is_its_roots(handle, n):
+    d = np.abs(inputs.normal(n, 1, 25))[:, 0] + 0.01
+    A = np.asfortranarray(np.diag(d))
+    for batched in (False, True):
+        dA, dB = cuda(A), cuda(np.ones((n, 1), order="F"))
+        if batched:
+            assert handle.hpd_solve_batched([dA], [dB]) == [0]
+        else:
+            handle.hpd_solve(dA, dB)
+        assert np.array_equal(np.tril(host(dA)), np.diag(np.sqrt(d)))
+
+
+# an infinite pivot: its root, zeros below it, and the others' solution with x = 0 there
+@pytest.mark.parametrize("n,at", [(40, 7), (40, 39), (100, 16), (300, 150)])
+def test_batched_hpd_infinite_diagonal_entry(handle, n, at):
+    A, B = inputs.spd_ggt(n, 26), inputs.normal(n, 2, 27)
+    G = A.copy(order="F")
+    G[at, at] = np.inf
+    dA, dB = cuda(G), cuda(B)
+    assert handle.hpd_solve_batched([dA], [dB]) == [0]
+    L, X = np.tril(host(dA)), host(dB)
+    assert L[at, at] == np.inf and (L[at + 1:, at] == 0.0).all()
+    assert (X[at] == 0.0).all()
+    keep = np.arange(n) != at
+    assert solve_bwd(A[np.ix_(keep, keep)], X[keep], B[keep]) <= 4
+
+
 # products of 32 columns (16-column panels: two sums) right of or left of the diagonal
 @pytest.mark.parametrize("n", [64, 320])
 @pytest.mark.parametrize("lower", [False, True])

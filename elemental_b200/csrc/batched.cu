@@ -68,24 +68,24 @@ constexpr int diag_ld(int NB) { return diag_w(NB) + 4; }
 
 // Shared-memory layout (bytes) for storage type T and panel width NB: the
 // panel P, the diagonal-block inverse / solve staging X (diag_w(NB) x diag_ld(NB)), the
-// diagonal block in FP64 while it is factored S (the same size), the
+// Cholesky's diagonal block in FP64 while it is factored S (the same size), the
 // left-looking dots Y (NB x kRC) and, for refined plans whose panel is
 // smaller than two right-hand-side chunks, the solution chunk BS.  The
 // solves' chunk R (and the refined plans' solution chunk otherwise) alias
 // the panel, which the factorization no longer needs by then.
 constexpr size_t kChunkBytes = (size_t)kRC * kBmaxN * 8;
-template <typename T, int NB>
+template <typename T, int NB, int KIND>
 struct BL {
   static constexpr int kXLD = diag_ld(NB);
   static constexpr size_t kPBytes = (size_t)NB * kPLD * sizeof(T);
   static constexpr bool kOwnBS = sizeof(T) == 4 && kPBytes < 2 * kChunkBytes;
   static constexpr size_t kOffX = (kPBytes + 15) & ~size_t(15);
   static constexpr size_t kOffS = kOffX + (size_t)diag_w(NB) * kXLD * 8;
-  static constexpr size_t kOffY = kOffS + (size_t)diag_w(NB) * kXLD * 8;
+  static constexpr size_t kOffY = kOffS + (KIND == 0 ? (size_t)diag_w(NB) * kXLD * 8 : 0);
   static constexpr size_t kOffB = kOffY + (size_t)NB * kRC * 8;
   static constexpr size_t kBytes = kOffB + (kOwnBS ? kChunkBytes : 0);
   static_assert(kPBytes >= kChunkBytes, "the solves' chunk aliases the panel");
-  static_assert((size_t)diag_w(NB) * kXLD * 8 >= 2 * 8 * (2 + NB / 2) * 16, "the panel's candidates (8 warps) fit S");
+  static_assert((size_t)diag_w(NB) * kXLD * 8 >= 2 * 8 * (2 + NB / 2) * 16, "the LU panel's candidates (8 warps) fit X");
 };
 
 struct BatchArgs {
@@ -101,6 +101,13 @@ struct BatchArgs {
 template <typename T> struct Pair2;
 template <> struct Pair2<double> { using type = double2; };
 template <> struct Pair2<float> { using type = float2; };
+
+// The GE kernels of FP64 plans keep panel rows in registers and a row's or a
+// tile's loads all in flight.  The refined plans' (two CTAs of 256 threads per
+// SM, 128 registers a thread) spill 920 bytes that way and take their loads as
+// they come: 296 systems, 4 right-hand sides, n = 64 371 -> 276 us, n = 512 8.96 -> 8.21 ms.
+template <typename T>
+constexpr bool kLoadAhead = sizeof(T) == 8;
 
 template <typename T>
 __device__ __forceinline__ double ldv(const T* p) { return (double)*p; }
@@ -224,9 +231,11 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
                                           int prow, int pcol, int mrows, int ncols, int pb) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double acc[2][4][4];
-  // C's loads are all in flight before the first is used (a test around each
-  // would run them one after the other)
+  // kAhead: C's and U's loads are all in flight before the first is used (a
+  // test around each would run them one after the other)
+  constexpr bool kAhead = kLoadAhead<T>;
   const bool full = cvec && prow + 32 <= mrows && pcol + 32 <= ncols;
+  auto pair = [&](int row, int col) { return kAhead ? full : cvec && row + 1 < mrows && col < ncols; };
 #pragma unroll
   for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -235,7 +244,7 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
       const int col = pcol + 8 * j + 2 * t + (r & 1);
       const T* cp = C + (long long)col * ldc + row;
       double c0 = 0.0, c1 = 0.0;
-      if (full) {
+      if (pair(row, col)) {
         ld_pair(cp, c0, c1);
       } else {
         if (row < mrows && col < ncols) c0 = ldv(cp);
@@ -244,24 +253,28 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
       acc[0][j][r] = -c0;
       acc[1][j][r] = -c1;
     }
-  double bf[NB / 8][4][2];  // U's fragments, in flight with C
-#pragma unroll
-  for (int ks = 0; ks < NB / 8; ++ks)
+  double bf[kAhead ? NB / 8 : 1][4][2];
+  auto load_u = [&](double (&f)[4][2], int ks) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int col = pcol + 8 * j + g;
       const T* up = U + (long long)col * ldu + ks * 8 + 2 * t;
-      bf[ks][j][0] = bf[ks][j][1] = 0.0;
-      if (full) {
-        ld_pair(up, bf[ks][j][0], bf[ks][j][1]);
+      f[j][0] = f[j][1] = 0.0;
+      if (kAhead ? full : cvec && col < ncols) {
+        ld_pair(up, f[j][0], f[j][1]);
       } else if (col < ncols) {
-        bf[ks][j][0] = ldv(up);
-        bf[ks][j][1] = ldv(up + 1);
+        f[j][0] = ldv(up);
+        f[j][1] = ldv(up + 1);
       }
     }
+  };
+  if (kAhead)
+#pragma unroll
+    for (int ks = 0; ks < NB / 8; ++ks) load_u(bf[ks], ks);
 #pragma unroll
   for (int ks = 0; ks < NB / 8; ++ks) {
     const int ke = ks * 8 + 2 * t;
+    if (!kAhead) load_u(bf[0], ks);
     double af[2][4];
     const int m0 = pb + prow + 2 * g;
     double x00, y00, x01, y01, x10, y10, x11, y11;
@@ -274,7 +287,7 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dmma_16x8x8(acc[i][j], af[i], bf[ks][j]);
+      for (int j = 0; j < 4; ++j) dmma_16x8x8(acc[i][j], af[i], bf[kAhead ? ks : 0][j]);
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -283,7 +296,7 @@ __device__ __forceinline__ void tile_gemm(T* C, long long ldc, bool cvec, const 
       const int row = prow + 2 * g + ((r >= 2) ? 16 : 0);
       const int col = pcol + 8 * j + 2 * t + (r & 1);
       T* cp = C + (long long)col * ldc + row;
-      if (full) {
+      if (pair(row, col)) {
         st_pair(cp, -acc[0][j][r], -acc[1][j][r]);
       } else {
         if (row < mrows && col < ncols) stv(cp, -acc[0][j][r]);
@@ -462,25 +475,93 @@ __device__ __forceinline__ int lu_panel_cols(T (&v)[kBmaxN / NT][NB], int (&pos)
   return 0;
 }
 
+// All b columns of lu_panel_smem with the rows left in shared memory.
+template <typename T, int NB, int NT>
+__device__ __forceinline__ int lu_panel_rows(int (&pos)[kBmaxN / NT], T* P, int m, int b, int* s_piv, double2* candb) {
+  constexpr int RPT = kBmaxN / NT, NW = NT / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  bool done[RPT];
+#pragma unroll
+  for (int t = 0; t < RPT; ++t) {
+    pos[t] = tid + t * NT;
+    done[t] = pos[t] >= m;
+  }
+#pragma unroll 1
+  for (int j = 0; j < b; ++j) {
+    double2* cand = candb + (j & 1) * NW;  // {|a|, position : row}
+    // this thread's candidate (a NaN is never one, as it never compares greater)
+    unsigned long long key = 0ull;
+    int kpos = kNoPos, krow = 0;
+#pragma unroll
+    for (int t = 0; t < RPT; ++t) {
+      if (done[t]) continue;
+      const int r = tid + t * NT;
+      const unsigned long long kk = abs_key(ldv(P + j * kPLD + r));
+      if (kk <= 0x7ff0000000000000ull && (kpos == kNoPos || kk > key || (kk == key && pos[t] < kpos))) {
+        key = kk;
+        kpos = pos[t];
+        krow = r;
+      }
+    }
+    const int wl = warp_argmax(key, kpos);
+    if (lane == max(wl, 0))
+      cand[warp] = make_double2(__longlong_as_double((long long)key), __hiloint2double(wl < 0 ? kNoPos : kpos, krow));
+    __syncthreads();
+    unsigned long long ck = 0ull;
+    int cpos = kNoPos;
+    if (lane < NW) {
+      const double2 h = cand[lane];
+      ck = (unsigned long long)__double_as_longlong(h.x);
+      cpos = __double2hiint(h.y);
+    }
+    const int wc = warp_argmax(ck, cpos);
+    if (wc < 0) return j + 1;
+    const double whd = cand[wc].y;
+    const int wpos = __double2hiint(whd), wrow = __double2loint(whd);
+    const double pv = ldv(P + j * kPLD + wrow);
+    if (pv == 0.0) return j + 1;
+    if (tid == 0) s_piv[j] = wpos;
+    const double rp = __drcp_rn(pv);
+#pragma unroll
+    for (int t = 0; t < RPT; ++t) {
+      const int r = tid + t * NT;
+      if (pos[t] == j) pos[t] = wpos;
+      if (r == wrow) {
+        done[t] = true;
+        pos[t] = j;
+      }
+      if (done[t]) continue;
+      const double l = ldv(P + j * kPLD + r) * rp;
+      stv(P + j * kPLD + r, l);
+      for (int c = j + 1; c < b; ++c)
+        stv(P + c * kPLD + r, fma(-l, ldv(P + c * kPLD + wrow), ldv(P + c * kPLD + r)));
+    }
+  }
+  return 0;
+}
+
 // LU with partial pivoting of the m x b panel in shared memory (lu::Panel,
 // LU/Panel.hpp:19-89: the entry of largest magnitude, the first in row
 // order on ties; zero pivot -> singular; a21 *= 1/alpha11; A22 -= a21 a12).
-// Every thread holds its rows (tid + t * NT) in registers; the chosen row is
-// marked done instead of swapped and every thread keeps the current position
-// of the rows it owns, so the sequential interchange semantics (position j <->
-// position p_j) hold and a column costs one CTA barrier; finished entries go
-// back to P.  (Updating the panel in shared memory took 2500 cycles per column
-// of a 32-wide panel.)  Afterwards the panel rows are permuted into position
-// order in place; s_mv receives the (from, to) row moves and s_piv[j] the
-// position swapped with j at step j.  candb: 2 * NT / 32 * (2 + NB / 2)
-// double2 of scratch.  Returns 0 or the 1-based column of a zero pivot
-// (CTA-uniform).
+// The chosen row is marked done instead of swapped and every thread keeps the
+// current position of the rows it owns (tid + t * NT), so the sequential
+// interchange semantics (position j <-> position p_j) hold and a column costs
+// one CTA barrier.  FP64 plans hold the rows in registers, finished entries go
+// back to P (updating the panel in shared memory took 2500 cycles per column
+// of a 32-wide panel); the refined plans' stay in P (kLoadAhead).  Afterwards
+// the panel rows are permuted into position order in place; s_mv receives the
+// (from, to) row moves and s_piv[j] the position swapped with j at step j.
+// candb: 2 * NT / 32 * (2 + NB / 2) double2 of scratch.  Returns 0 or the
+// 1-based column of a zero pivot (CTA-uniform).
 template <typename T, int NB, int NT>
 __device__ int lu_panel_smem(T* P, int m, int b, int* s_piv, int* s_mv, int* s_nmv, double2* candb) {
   constexpr int RPT = kBmaxN / NT;
   const int tid = threadIdx.x;
   int pos[RPT];
-  {
+  if constexpr (!kLoadAhead<T>) {
+    const int f = lu_panel_rows<T, NB, NT>(pos, P, m, b, s_piv, candb);
+    if (f) return f;
+  } else {
     T v[RPT][NB];
     bool done[RPT];
 #pragma unroll
@@ -627,7 +708,7 @@ __device__ int lu_factor(T* F, long long ldf, int n, T* P, const BWork& w, doubl
       for (int r = tid; r < m; r += NT) cp_async_el(&P[c * kPLD + r], &F[(long long)(k0 + c) * ldf + k0 + r]);
     cp_async_wait_all();
     __syncthreads();
-    const int f = lu_panel_smem<T, NB, NT>(P, m, b, w.piv, w.mv, w.nmv, reinterpret_cast<double2*>(w.S));
+    const int f = lu_panel_smem<T, NB, NT>(P, m, b, w.piv, w.mv, w.nmv, reinterpret_cast<double2*>(w.X));
     if (f) {
       __syncthreads();
       return k0 + f;
@@ -717,46 +798,69 @@ __device__ int lu_factor(T* F, long long ldf, int n, T* P, const BWork& w, doubl
 // block's right-hand side rq (bi entries, shared): the unit lower part (UNIT:
 // rq[i] + sum_{k < i} X(i, k) rq[k]), the lower part (k <= i), the upper part
 // (upper: k >= i) or, TRANS, the lower part's transpose (sum_{k >= i} X(k, i)
-// rq[k]).  All NB loads of the row are in flight at once (a loop over the row
-// waited for L2 every few entries).
-template <int NB, bool UNIT, bool TRANS>
+// rq[k]).  AHEAD: all NB loads of the row are in flight at once (a loop over
+// the row waits for L2 every few entries).
+template <int NB, bool UNIT, bool TRANS, bool AHEAD>
 __device__ __forceinline__ double block_row(const double* X, int i, int bi, const double* rq, bool upper = false) {
-  auto in = [&](int k) { return k < bi && (UNIT ? k < i : (TRANS || upper) ? k >= i : k <= i); };
+  [[maybe_unused]] auto in = [&](int k) { return k < bi && (UNIT ? k < i : (TRANS || upper) ? k >= i : k <= i); };
   if (i >= bi) return 0.0;
-  double x[NB];
+  if constexpr (!AHEAD) {
+    const bool up = TRANS || upper;
+    double s = UNIT ? rq[i] : 0.0;
+    for (int k = up ? i : 0, end = up ? bi : UNIT ? i : i + 1; k < end; ++k)
+      s = fma(X[TRANS ? k + i * NB : i + k * NB], rq[k], s);
+    return s;
+  } else {
+    double x[NB];
 #pragma unroll
-  for (int k = 0; k < NB; ++k) x[k] = in(k) ? X[TRANS ? k + i * NB : i + k * NB] : 0.0;
-  double s0 = UNIT ? rq[i] : 0.0, s1 = 0.0;
+    for (int k = 0; k < NB; ++k) x[k] = in(k) ? X[TRANS ? k + i * NB : i + k * NB] : 0.0;
+    double s0 = UNIT ? rq[i] : 0.0, s1 = 0.0;
 #pragma unroll
-  for (int k = 0; k < NB; k += 2) {  // an entry outside the part never meets rq (which may not be finite)
-    if (in(k)) s0 = fma(x[k], rq[k], s0);
-    if (in(k + 1)) s1 = fma(x[k + 1], rq[k + 1], s1);
+    for (int k = 0; k < NB; k += 2) {  // an entry outside the part never meets rq (which may not be finite)
+      if (in(k)) s0 = fma(x[k], rq[k], s0);
+      if (in(k + 1)) s1 = fma(x[k + 1], rq[k + 1], s1);
+    }
+    return s0 + s1;
   }
-  return s0 + s1;
 }
 
 // R[q][r] -= sum_k F(r, k) stage[k + q NB] over the block's bi columns (F at
-// its first column), rows r0 <= r < r1; all of a row's loads in flight.  The
+// its first column), rows r0 <= r < r1; AHEAD: all of a row's loads in flight.  The
 // products are summed before they meet R (GE, mean backward error at n = 512:
 // 2.8e-16 with one of the two sums started at R, 2.3e-16 this way).
-template <typename T, int NB, int NT>
+template <typename T, int NB, int NT, bool AHEAD>
 __device__ __forceinline__ void rows_update(const T* F, long long ldf, int bi, int r0, int r1, int nr,
                                             const double* stage, double* R) {
   for (int r = r0 + (int)threadIdx.x; r < r1; r += NT) {
-    T l[NB];
+    if constexpr (!AHEAD) {
+      double acc[kRC];
 #pragma unroll
-    for (int k = 0; k < NB; ++k) l[k] = k < bi ? F[(long long)k * ldf + r] : T(0);
+      for (int q = 0; q < kRC; ++q) acc[q] = 0.0;
+      for (int k = 0; k < bi; ++k) {
+        const double l = ldv(F + (long long)k * ldf + r);
 #pragma unroll
-    for (int q = 0; q < kRC; ++q)
-      if (q < nr) {
-        double a0 = 0.0, a1 = 0.0;
-#pragma unroll
-        for (int k = 0; k < NB; k += 2) {
-          a0 = fma((double)l[k], stage[k + q * NB], a0);
-          a1 = fma((double)l[k + 1], stage[k + 1 + q * NB], a1);
-        }
-        R[q * kBmaxN + r] -= a0 + a1;
+        for (int q = 0; q < kRC; ++q)
+          if (q < nr) acc[q] = fma(l, stage[k + q * NB], acc[q]);
       }
+#pragma unroll
+      for (int q = 0; q < kRC; ++q)
+        if (q < nr) R[q * kBmaxN + r] -= acc[q];
+    } else {
+      T l[NB];
+#pragma unroll
+      for (int k = 0; k < NB; ++k) l[k] = k < bi ? F[(long long)k * ldf + r] : T(0);
+#pragma unroll
+      for (int q = 0; q < kRC; ++q)
+        if (q < nr) {
+          double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+          for (int k = 0; k < NB; k += 2) {
+            a0 = fma((double)l[k], stage[k + q * NB], a0);
+            a1 = fma((double)l[k + 1], stage[k + 1 + q * NB], a1);
+          }
+          R[q * kBmaxN + r] -= a0 + a1;
+        }
+    }
   }
 }
 
@@ -771,6 +875,7 @@ __device__ void solve_smem(const T* F, long long ldf, int n, int nr, const doubl
                            const BWork& w) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = NT / 32;
+  constexpr bool kAhead = !LU || kLoadAhead<T>;
   double* stage = w.X;  // NB x nr
   const int nblk = (n + NB - 1) / NB;
   for (int ib = 0; ib < nblk; ++ib) {
@@ -792,12 +897,12 @@ __device__ void solve_smem(const T* F, long long ldf, int n, int nr, const doubl
     const double* Xi = Xg + (size_t)ib * NB * NB;
     for (int e = tid; e < NB * nr; e += NT) {
       const int i = e % NB, q = e / NB;
-      stage[e] = block_row<NB, LU, false>(Xi, i, bi, R + q * kBmaxN + i0);
+      stage[e] = block_row<NB, LU, false, kAhead>(Xi, i, bi, R + q * kBmaxN + i0);
     }
     __syncthreads();
     for (int e = tid; e < NB * nr; e += NT)
       if (e % NB < bi) R[(e / NB) * kBmaxN + i0 + e % NB] = stage[e];
-    rows_update<T, NB, NT>(F + (long long)i0 * ldf, ldf, bi, i0 + bi, n, nr, stage, R);
+    rows_update<T, NB, NT, kAhead>(F + (long long)i0 * ldf, ldf, bi, i0 + bi, n, nr, stage, R);
     __syncthreads();
   }
   for (int ib = nblk - 1; ib >= 0; --ib) {
@@ -845,12 +950,12 @@ __device__ void solve_smem(const T* F, long long ldf, int n, int nr, const doubl
     }
     for (int e = tid; e < NB * nr; e += NT) {
       const int i = e % NB, q = e / NB;
-      stage[e] = block_row<NB, false, !LU>(Xi, i, bi, R + q * kBmaxN + i0, LU);
+      stage[e] = block_row<NB, false, !LU, kAhead>(Xi, i, bi, R + q * kBmaxN + i0, LU);
     }
     __syncthreads();
     for (int e = tid; e < NB * nr; e += NT)
       if (e % NB < bi) R[(e / NB) * kBmaxN + i0 + e % NB] = stage[e];
-    if (LU) rows_update<T, NB, NT>(F + (long long)i0 * ldf, ldf, bi, 0, i0, nr, stage, R);
+    if (LU) rows_update<T, NB, NT, kAhead>(F + (long long)i0 * ldf, ldf, bi, 0, i0, nr, stage, R);
     __syncthreads();
   }
 }
@@ -1003,7 +1108,7 @@ __device__ int refine_chunk(const double* A, long long lda, int n, double* B, lo
 template <typename T, int NB, int NT, int MINB, int KIND>
 __global__ void __launch_bounds__(NT, MINB) batched_kernel(BatchArgs args) {
   extern __shared__ __align__(16) unsigned char sm_dyn[];
-  using LY = BL<T, NB>;
+  using LY = BL<T, NB, KIND>;
   constexpr bool kRefined = sizeof(T) == 4;
   constexpr bool kHPD = KIND == 0;
   __shared__ double s_rd[32];
@@ -1115,12 +1220,12 @@ __global__ void batch_backup_kernel(const BatchItem* items, int count, double* b
 typedef void (*BatchKernel)(BatchArgs);
 struct Variant {
   BatchKernel kern[2];
-  size_t smem;
+  size_t smem[2];
   int nb, nt;
 };
 
 #define EGPU_BVAR(T, NB, NT, MINB) \
-  { {batched_kernel<T, NB, NT, MINB, 0>, batched_kernel<T, NB, NT, MINB, 1>}, BL<T, NB>::kBytes, NB, NT }
+  { {batched_kernel<T, NB, NT, MINB, 0>, batched_kernel<T, NB, NT, MINB, 1>}, {BL<T, NB, 0>::kBytes, BL<T, NB, 1>::kBytes}, NB, NT }
 
 // FP64 plans: (panel 32, 256 threads, one CTA per SM), (16, 256, two per SM),
 // (16, 128, two per SM).  Refined plans: (32, 256, two per SM), (16, 256, two
@@ -1149,9 +1254,9 @@ static int variant_prepare(const Variant& v, int kind, int* per_sm) {
     *per_sm = *slot;
     return EGPU_OK;
   }
-  EGPU_CUDA_TRY(cudaFuncSetAttribute(v.kern[kind], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
+  EGPU_CUDA_TRY(cudaFuncSetAttribute(v.kern[kind], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem[kind]));
   int occ = 0;
-  EGPU_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, v.kern[kind], v.nt, v.smem));
+  EGPU_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, v.kern[kind], v.nt, v.smem[kind]));
   *per_sm = std::max(1, std::min(occ, kMaxPerSM));
   if (slot) *slot = *per_sm;
   return EGPU_OK;
@@ -1225,7 +1330,7 @@ int egpu_batched_launch(int kind, cudaStream_t st, int sm_count, int count, cons
     for (int i = 0; i < count; ++i) flops += (kind == 0 ? 1.0 / 3.0 : 2.0 / 3.0) * (double)n[i] * n[i] * n[i];
     TraceMark tm(st, kTraceOther, flops, 0.0);
     BatchArgs a{d_items, count, d_counter, d_info, nullptr, d_scr};
-    v.kern[kind]<<<grid, v.nt, v.smem, st>>>(a);
+    v.kern[kind]<<<grid, v.nt, v.smem[kind], st>>>(a);
     count_launch();
   }
   EGPU_CUDA_TRY(cudaGetLastError());
@@ -1353,7 +1458,7 @@ static int plan_launch(BatchPlan* p, cudaStream_t st, int cls, int beg, int end,
   }
   TraceMark tm(st, kTraceOther, flops, 0.0);
   BatchArgs a{p->d_items + beg, end - beg, p->d_counter + cls, p->d_info, p->d_iters, p->d_scr};
-  v.kern[p->kind]<<<grid, v.nt, v.smem, st>>>(a);
+  v.kern[p->kind]<<<grid, v.nt, v.smem[p->kind], st>>>(a);
   count_launch();
   EGPU_CUDA_TRY(cudaGetLastError());
   return EGPU_OK;

@@ -1262,15 +1262,24 @@ static int variant_prepare(const Variant& v, int kind, int* per_sm) {
   return EGPU_OK;
 }
 
-// The shape used without tuning, from the kind and the largest order.  FP64 HPD:
-// two CTAs per SM with 16-wide panels, whose chains overlap (4096 systems, n =
-// 32..512: 9.9 ms against 11.2 with one CTA and 32-wide panels; n = 512 alone
-// 3.99 and 4.03).  FP64 GE: the same with 128 threads while the systems are
-// small (n <= 256: 5.7 against 6.6 ms; n <= 64 1.06 and 1.87), above that one CTA
-// with 32-wide panels, which moves the trailing matrix half as often (what the
-// autotuner picks at n = 512 too).
-static int default_variant(int kind, int precision, int nmax) {
-  if (precision != 0) return 0;
+// The shape used without tuning, from the kind and the orders (largest first).
+// Where the systems are no more work than one CTA per SM takes in the largest
+// one's time (work ~ n^2), that system's chain counts, and 32-wide panels have
+// the shorter one.  us, 32-wide / two CTAs per SM with 16-wide panels: 148 HPD
+// systems of n = 128 106 / 139, 512 903 / 1642, 400 of n = 32..512 1010 / 1749; 148 GE
+// systems (128 threads) of n = 128 186 / 246, 256 490 / 797.  (Orders up to 16 leave
+// half of a 32-wide panel empty: GE 31 / 27.)
+// Above that FP64 HPD takes the 16-wide shape, whose two chains overlap (200 of
+// n = 128 205 / 139, 256 485 / 381, 512 1671 / 1714; 1500 of n = 32..512 3721 / 3291),
+// and FP64 GE the same with 128 threads while the systems are small (200 of n =
+// 128 356 / 248, 256 954 / 836), above that the 32-wide one, which moves the
+// trailing matrix half as often (200 of n = 512 3.7 / 4.3 ms).
+static int default_variant(int kind, int precision, const std::vector<BatchItem>& items, int sm_count) {
+  if (precision != 0 || items.empty()) return 0;
+  const double nmax = items[0].n;
+  double work = 0.0;
+  for (const BatchItem& it : items) work += (double)it.n * it.n;
+  if (nmax > 16 && work <= (double)sm_count * nmax * nmax) return 0;
   if (kind == 0) return 1;
   return nmax <= 256 ? 2 : 0;
 }
@@ -1305,7 +1314,7 @@ int egpu_batched_launch(int kind, cudaStream_t st, int sm_count, int count, cons
     items[i].id = i;
   }
   sort_items(items);
-  const Variant& v = kVariants[0][default_variant(kind, 0, count > 0 ? items[0].n : 0)];
+  const Variant& v = kVariants[0][default_variant(kind, 0, items, sm_count)];
   int per_sm = 1;
   BTRY(variant_prepare(v, kind, &per_sm));
   const int grid = std::max(1, std::min(std::min(per_sm, 2) * sm_count, count));
@@ -1382,7 +1391,7 @@ static int plan_single_shape(BatchPlan* p, int var) {
 }
 
 static int plan_default_shape(BatchPlan* p) {
-  return plan_single_shape(p, default_variant(p->kind, p->precision, p->count > 0 ? p->items[0].n : 0));
+  return plan_single_shape(p, default_variant(p->kind, p->precision, p->items, p->sm_count));
 }
 
 int batch_plan_create(int device, int sm_count, int kind, int precision, int count, const int* n, const int* nrhs,

@@ -259,6 +259,22 @@ def test_batched_block_edges(handle, sizes):
             assert solve_bwd(a, host(x), b) <= 4
 
 
+@pytest.mark.parametrize("panel,threads", [(32, 256), (16, 256), (16, 128)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_batched_block_edges_in_every_shape(handle, kind, panel, threads):
+    sizes = (1, 15, 16, 17, 31, 32, 33, 64, 257, 300, 512)
+    As = [inputs.spd_ggt(n, 60 + n) if kind == 0 else inputs.uniform(n, n, 60 + n) for n in sizes]
+    Bs = [inputs.normal(n, 1 + i % 9, 80 + n) for i, n in enumerate(sizes)]
+    dA, dB = [cuda(a) for a in As], [cuda(b) for b in Bs]
+    plan = eg.BatchPlan(handle, kind, dA, dB)
+    plan.set_shape(panel, threads)
+    plan.run()
+    assert plan.info() == [0] * len(sizes)
+    for a, b, x in zip(As, Bs, dB):
+        assert solve_bwd(a, host(x), b) <= 4
+    plan.close()
+
+
 def test_batched_lu_ties_and_singular_column(handle):
     A = np.asfortranarray(np.sign(inputs.uniform(40, 40, 18)))
     Z = inputs.uniform(40, 40, 19)

@@ -128,12 +128,20 @@ __device__ __forceinline__ void small_stage(double* S, const double* G, long lon
   }
 }
 
-template <bool AK, bool BK, int TM, int TN>
+// U: the k loop's unrolling.  2 takes up to 70 registers, three CTAs to an SM,
+// which is what the operands leave room for from K = 128 on (us, U = 1 / 2, NORMAL,
+// NORMAL, 768^2 14.5 / 12.4, 1216^2 24.7 / 22.7); with K <= 64 and U = 1 there are five
+// (8.3 / 10.4 at 768^2, K = 64).
+template <bool AK, bool BK, int TM, int TN, int U>
 __global__ void __launch_bounds__(256) dgemm_small_kernel(const SmallParams p) {
   extern __shared__ __align__(16) double ss[];
   constexpr int TILES = (TM / 16) * (TN / 8), PER = TILES / 8;  // 16 x 8 DMMA tiles per warp
   static_assert(TILES % 8 == 0, "eight warps");
-  __shared__ int s_go;
+  // an earlier step failed: the CTA takes one thread's reading (another stream
+  // may set the status meanwhile), which comes in with the copies.  (Through a
+  // shared word it cost 10 to 30% of 500 CTAs and more at K = 128.)
+  bool bad = false;
+  if (threadIdx.x == 0) bad = p.status != nullptr && ((const volatile DevStatus*)p.status)->code != 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * TM, col0 = blockIdx.y * TN;
@@ -155,12 +163,8 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(const SmallParams p) {
       cc[j][r] = v ? p.C[m + (long long)n * p.ldc] : 0.0;
       acc[j][r] = 0.0;
     }
-  // an earlier step failed: the CTA takes one thread's reading (another stream
-  // may set the status meanwhile), made while the copies are in flight
-  if (threadIdx.x == 0) s_go = p.status == nullptr || ((const volatile DevStatus*)p.status)->code == 0;
   cp_async_wait_all();
-  __syncthreads();
-  if (!s_go) return;
+  if (__syncthreads_or(bad)) return;
   const int as = AK ? 1 : small_ld(TM), am = AK ? KP + 4 : 1;  // k and row strides
   const int bs = BK ? 1 : small_ld(TN), bn = BK ? KP + 4 : 1;
   const double* pa = sA + (16 * rt + g) * am + t * as;
@@ -179,7 +183,7 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(const SmallParams p) {
     }
   };
   int k0 = 0;
-#pragma unroll 2
+#pragma unroll U
   for (; k0 + 8 < KP; k0 += 16) {
     step(acc, k0);
     step(acc2, k0 + 8);
@@ -196,9 +200,9 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(const SmallParams p) {
     }
 }
 
-template <bool AK, bool BK, int TM, int TN>
+template <bool AK, bool BK, int TM, int TN, int U>
 static cudaError_t launch_small_variant(cudaStream_t st, const SmallParams& p) {
-  auto kern = dgemm_small_kernel<AK, BK, TM, TN>;
+  auto kern = dgemm_small_kernel<AK, BK, TM, TN, U>;
   constexpr int kMax = 200 * 1024;
   static unsigned attr_mask = 0;  // per template instance, one bit per device
   int dev = 0;
@@ -218,12 +222,12 @@ static cudaError_t launch_small_variant(cudaStream_t st, const SmallParams& p) {
   return cudaGetLastError();
 }
 
-template <int TM, int TN>
+template <int TM, int TN, int U = 2>
 static cudaError_t launch_small_tile(cudaStream_t st, bool ak, bool bk, const SmallParams& p) {
-  if (ak && bk) return launch_small_variant<true, true, TM, TN>(st, p);
-  if (ak) return launch_small_variant<true, false, TM, TN>(st, p);
-  if (bk) return launch_small_variant<false, true, TM, TN>(st, p);
-  return launch_small_variant<false, false, TM, TN>(st, p);
+  if (ak && bk) return launch_small_variant<true, true, TM, TN, U>(st, p);
+  if (ak) return launch_small_variant<true, false, TM, TN, U>(st, p);
+  if (bk) return launch_small_variant<false, true, TM, TN, U>(st, p);
+  return launch_small_variant<false, false, TM, TN, U>(st, p);
 }
 
 // Do two column-major views share an element?  Views with the same leading
@@ -278,6 +282,7 @@ static int launch_dgemm_small(cudaStream_t st, bool a_kmajor, bool b_kmajor, int
   else if (alias_a) e = launch_small_tile<32, 128>(st, a_kmajor, b_kmajor, p);
   else if (alias_b && N <= 16 * 148) e = launch_small_tile<128, 16>(st, a_kmajor, b_kmajor, p);
   else if (alias_b) e = launch_small_tile<128, 32>(st, a_kmajor, b_kmajor, p);
+  else if (K <= 64) e = launch_small_tile<32, 32, 1>(st, a_kmajor, b_kmajor, p);
   else e = launch_small_tile<32, 32>(st, a_kmajor, b_kmajor, p);
   if (e != cudaSuccess) {
     set_last_error(e, "dgemm_small launch", __FILE__, __LINE__);

@@ -54,6 +54,17 @@ bool make_tma_2d(CUtensorMap* m, int dtype, const void* base, uint64_t inner, ui
   return r == CUDA_SUCCESS;
 }
 
+static int sm_count_of_current_device() {
+  static int cache[32] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 32 && cache[dev] > 0) return cache[dev];
+  int n = 0;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  if (dev >= 0 && dev < 32) cache[dev] = n;
+  return n;
+}
+
 bool tma_compatible(const void* p, long long ld) {
   return (reinterpret_cast<uintptr_t>(p) % 16 == 0) && (ld % 2 == 0) && ld > 0;
 }
@@ -262,14 +273,24 @@ static int launch_dgemm_small(cudaStream_t st, bool a_kmajor, bool b_kmajor, int
   // (column n of C is column n of op(B)^T)
   if (alias_a && !(C == A && ldc == lda && !a_kmajor && N <= 128 && K <= 128)) return EGPU_ERR_UNSUPPORTED;
   if (alias_b && !(C == B && ldc == ldb && b_kmajor && M <= 128 && K <= 128)) return EGPU_ERR_UNSUPPORTED;
+  const int sms = sm_count_of_current_device();
   const long long t32 = (long long)((M + 31) / 32) * ((N + 31) / 32);
-  // where the engine, whose tiles need half the operand traffic, catches up (K =
-  // 128, us, engine / this form): 1600 tiles of 32 x 32 (1280^2) 28.9 / 22.8,
-  // 2304 tiles (1536^2) 28.9 / 30.9; in place one wave of CTAs (M = 2048: 22 /
-  // 10; the Cholesky at n = 16384 0.6% slower with the whole range of M here)
-  if (!alias_a && !alias_b && t32 / (tri ? 2 : 1) > 1480) return EGPU_ERR_UNSUPPORTED;
-  if (alias_a && M > 32 * 148) return EGPU_ERR_UNSUPPORTED;
-  if (alias_b && N > 32 * 148) return EGPU_ERR_UNSUPPORTED;
+  // Out of place up to where the engine, whose tiles need half the operand
+  // traffic, catches up.  This form's time over the engine's, 148 SMs, best and
+  // worst layout (MN-major both, K-major both): K = 64, 1444 tiles of 32 x 32
+  // (1216^2) 0.82 and 0.84, 1936 1.00 and 1.11; K = 128, 1444 0.72 and 0.90, 1764 0.86 and
+  // 1.04, 2304 1.06 and 1.32; K = 256, MN-major, 784 0.88, 1444 0.98.  K-major operands
+  // cost more with K, and the engine has one CTA to an SM up to 148 of its tiles:
+  // both K-major 576 tiles 0.84 at K = 192 and 1.01 at 256, 1024 1.32 and 1.69, 1444 1.00
+  // and 1.36; one K-major, K = 256, 576 0.78, 784 1.12, 1444 1.10.  At most 64 rows or
+  // columns leave half of the engine's tile empty: 64 x 16384, K = 256, 0.68 to 1.00.
+  // In place one wave of CTAs (M = 2048: 22 us in the engine, 10 here; the
+  // Cholesky at n = 16384 0.6% slower with the whole range of M here).
+  const bool long_k = a_kmajor && b_kmajor ? K > 128 : (a_kmajor || b_kmajor) && K > 192;
+  const int per_sm = long_k && std::min(M, N) > 64 ? 4 : 10;
+  if (!alias_a && !alias_b && t32 / (tri ? 2 : 1) > (long long)per_sm * sms) return EGPU_ERR_UNSUPPORTED;
+  if (alias_a && M > 32 * sms) return EGPU_ERR_UNSUPPORTED;
+  if (alias_b && N > 32 * sms) return EGPU_ERR_UNSUPPORTED;
   SmallParams p;
   p.A = A; p.B = B; p.C = C; p.lda = lda; p.ldb = ldb; p.ldc = ldc;
   p.M = M; p.N = N; p.K = K; p.tri = tri; p.alpha = alpha; p.beta = beta; p.status = status;
@@ -278,9 +299,9 @@ static int launch_dgemm_small(cudaStream_t st, bool a_kmajor, bool b_kmajor, int
   TraceMark tm(st, beta == 0.0 ? kTraceTrsm : kTraceUpdate, 2.0 * entries * K,
                8.0 * ((double)M * K + (double)N * K + (beta == 0.0 ? 1.0 : 2.0) * entries));
   cudaError_t e;
-  if (alias_a && M <= 16 * 148) e = launch_small_tile<16, 128>(st, a_kmajor, b_kmajor, p);
+  if (alias_a && M <= 16 * sms) e = launch_small_tile<16, 128>(st, a_kmajor, b_kmajor, p);
   else if (alias_a) e = launch_small_tile<32, 128>(st, a_kmajor, b_kmajor, p);
-  else if (alias_b && N <= 16 * 148) e = launch_small_tile<128, 16>(st, a_kmajor, b_kmajor, p);
+  else if (alias_b && N <= 16 * sms) e = launch_small_tile<128, 16>(st, a_kmajor, b_kmajor, p);
   else if (alias_b) e = launch_small_tile<128, 32>(st, a_kmajor, b_kmajor, p);
   else if (K <= 64) e = launch_small_tile<32, 32, 1>(st, a_kmajor, b_kmajor, p);
   else e = launch_small_tile<32, 32>(st, a_kmajor, b_kmajor, p);
@@ -344,10 +365,16 @@ int launch_dgemm(cudaStream_t st, bool a_kmajor, bool b_kmajor, int M, int N, in
   const double bytes = 8.0 * ((double)M * K + (double)N * K + (beta == 0.0 ? 1.0 : 2.0) * entries);
   TraceMark tm(st, beta == 0.0 ? kTraceTrsm : kTraceUpdate, flops, bytes);
   cudaError_t e;
-  // warps of 64 x 32 for long k loops that fill the chip several times (the
-  // deferred Herk of the grouped Cholesky), of 32 x 32 for the rest: n = 8192,
-  // C full NT, K = 128 0.73 and 0.65 ms, 512 2.31 and 2.30, 2048 8.47 and 8.70
-  const bool big = K >= 1024 && nblocks >= 1184;  // four CTAs a slot on 148 SMs
+  // Warps of 64 x 32 for long k loops whose last wave leaves most SMs with two
+  // CTAs (the main loop counts); of 32 x 32 for short ones (the epilogue counts)
+  // and where the last wave leaves one CTA to an SM, which four of the larger
+  // warps do not fill.  C full, NT, time with 64 x 32 over that with 32 x 32, 296 CTAs
+  // at once: n = 1500 (288 CTAs) K = 128 1.01, 384 0.92, 4096 0.89; n = 2048 (512) K =
+  // 256 0.98, 384 0.96, 4096 0.92; n = 3000 (1128) K = 384 1.04, 512 1.01, 4096 0.94; n =
+  // 8192 K = 128 1.23, 512 1.02, 2048 1.01; but n = 1000 (128) 1.09, n = 1800 (435)
+  // 1.17 and n = 3500 (1540) 1.05 to 1.08 at every K >= 512
+  const long long slots = 2ll * sm_count_of_current_device(), last = nblocks % slots;
+  const bool big = K >= (nblocks <= 2 * slots ? 384 : 512) && (last == 0 || 2 * last > slots);
   if (wide) {
     if (!b_kmajor) e = launch_variant<false, false, 2, 4, 2>(st, ma, mb, p, nblocks);
     else e = launch_variant<false, true, 2, 4, 2>(st, ma, mb, p, nblocks);

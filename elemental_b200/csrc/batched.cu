@@ -343,8 +343,9 @@ __device__ int diag_chol_warp(T* P, int b, double* S, double* X, double* col) {
   if (f) return f;
   if (lane < b) {
 #pragma unroll 8
-    for (int c = 0; c < NB; ++c)  // c <= lane < b <= NB
-      if (c <= lane) stv(P + c * kPLD + lane, S[lane + c * LD]);
+    for (int c = 0; c < NB; ++c)  // c < lane < b <= NB
+      if (c < lane) stv(P + c * kPLD + lane, S[lane + c * LD]);
+    stv(P + lane * kPLD + lane, sqrt(S[lane + lane * LD]));
   }
   __syncwarp();
   return 0;

@@ -100,9 +100,10 @@ __device__ __forceinline__ void warp_chol16_cols(double (&z)[16], double& d, dou
 // column is one reciprocal square root, one multiply and one FMA (55 + 23 + 23
 // cycles here): the broadcast precedes the square root, and the next pivot is
 // formed by every lane from a copy of a_{j+1,j+1} fetched beforehand.  The
-// diagonal itself is each lane's root of its own pivot, all 16 side by side at
-// the end: d times the reciprocal root is up to an ulp off, and NaN for an
-// infinite pivot (whose column is 0 and whose row of the inverse is 0).
+// diagonal keeps the pivots: who stores the factor takes their roots, all of a
+// block's side by side (here, one root per leaf, 230 cycles).  d times the
+// reciprocal root would be up to an ulp off, and NaN for an infinite pivot
+// (whose column is 0 and whose row of the inverse is 0).
 // Measured per block, alone on the SM: 7000 cycles with the reciprocal, the
 // root and the failure test in the chain one after the other.
 // buf: 32 doubles of shared memory, 16-byte aligned, of this warp.
@@ -118,7 +119,7 @@ __device__ inline int warp_chol16(double* S, int lds, int o, double* X, int ldx,
   int fail = 0;
   warp_chol16_cols<15>(z, d, mine, fail, 0, inv, i, Sd, lds, X + i * ldx, buf);
   warp_chol16_cols<7>(z, d, mine, fail, 8, inv, i, Sd, lds, X + i * ldx, buf);
-  if (!inv) Sd[i * lds] = sqrt(mine);
+  if (!inv) Sd[i * lds] = mine;
   __syncwarp();
   return fail;
 }
@@ -372,9 +373,9 @@ __device__ inline void smem_l21_inplace(double* P, int m2, const double* X11) {
 // factored and inverted by one warp (X11 into Xl), L21 = A21 X11^T and the
 // trailing update A22 -= L21 L21^T on the tensor cores.  Look-ahead: while
 // warps 1.. update the rest of A22, warp 0 updates the next diagonal leaf
-// first and factors it.  Returns 0 or the 1-based column of a non-positive
-// pivot (uniform).
-__device__ inline int smem_chol_dmma(double* S, int bp, double* Xl, double* /*T*/) {
+// first and factors it.  The diagonal keeps the pivots (see warp_chol16).
+// Returns 0 or the 1-based column of a non-positive pivot (uniform).
+__device__ inline int smem_chol_dmma(double* S, int bp, double* Xl) {
   __shared__ int s_fail;
   __shared__ __align__(16) double s_col[32];
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;

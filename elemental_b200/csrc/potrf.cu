@@ -64,12 +64,16 @@ __global__ void __launch_bounds__(kDiagThreads) potrf_diag_kernel(double* A, lon
   double* T = Xl + 8 * 16 * kLeafLD;
   const int bp = pad16_identity(S, b);
   __syncthreads();
-  const int f = smem_chol_dmma(S, bp, Xl, T);
+  const int f = smem_chol_dmma(S, bp, Xl);
   if (f) {
     if (tid == 0) set_status(st, kNotHPD, col_base + f);
     return;
   }
-  if (store_factor) tri_store(S, A, lda, b, UPLO != EGPU_LOWER, false);
+  if (store_factor) {
+    if (tid < b) S[tid + tid * kLDS] = sqrt(S[tid + tid * kLDS]);  // b <= 128 < kDiagThreads
+    __syncthreads();
+    tri_store(S, A, lda, b, UPLO != EGPU_LOWER, false);
+  }
   if (W == nullptr) return;  // the last block: no panel to multiply (the inverse is 12 of 47 us)
   __syncthreads();
   smem_trinv_dmma(S, bp, Xl, T);
@@ -141,7 +145,7 @@ __global__ void __launch_bounds__(kDiagThreads) potrf_diag_f32_kernel(const __gr
   double* T = Xl + 8 * 16 * kLeafLD;
   const int bp = pad16_identity(S, b);
   __syncthreads();
-  const int f = smem_chol_dmma(S, bp, Xl, T);
+  const int f = smem_chol_dmma(S, bp, Xl);
   if (f) {
     if (tid == 0) set_status(st, kNotHPD, col_base + f);
     return;

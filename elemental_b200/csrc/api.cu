@@ -549,8 +549,8 @@ int gesv_core(egpu_context* h, int n, int nrhs, double* A, long long lda, double
   int rc = read_status(h, &info);
   if (rc != EGPU_OK) return rc;
   if (nrhs == 0) return EGPU_OK;
-  // few right-hand sides: one launch (n = 777, 5 right-hand sides: 0.17 ms as
-  // one multiply and one update per block, 0.08 this way)
+  // few right-hand sides: one launch (n = 777, 5 right-hand sides, traced: 0.33 ms
+  // as one multiply and one update per block, 0.08 this way)
   if (skinny_ok(h, nrhs, A, lda, B, ldb)) return skinny_single(h, n, nrhs, A, lda, B, ldb, {EGPU_UPPER, 0, 1, 0});
   return trsm_core(h, EGPU_LEFT, EGPU_UPPER, 0, 0, n, nrhs, 1.0, A, lda, B, ldb);
 }

@@ -6,10 +6,10 @@
 // queue (largest first) with an atomic counter, so the uneven sizes balance
 // across the SMs.  Per system the CTA runs the blocked right-looking
 // algorithm with an NB-wide panel held in shared memory:
-//   * Cholesky: the diagonal block is factored by one warp with the block in
-//     registers (lane = row, shuffles along the column, no CTA barrier per
-//     column); its inverse is formed by the same warp with a short dependent
-//     chain (reciprocal diagonal, right-looking column accumulation); the
+//   * Cholesky: the diagonal block is factored and inverted by one warp in
+//     shared memory, in 16-column leaves (warp_chol16: a block's rows and the
+//     identity's columns go through the same steps, no CTA barrier per column)
+//     with the 16 x 16 products between them on DMMA; the
 //     panel solve is a multiply by that inverse; the trailing update runs on
 //     the FP64 tensor cores (DMMA m16n8k8, 32x32 warp tiles) over the
 //     system's trailing matrix in global memory.
@@ -105,7 +105,7 @@ template <> struct Pair2<float> { using type = float2; };
 // The GE kernels of FP64 plans keep panel rows in registers and a row's or a
 // tile's loads all in flight.  The refined plans' (two CTAs of 256 threads per
 // SM, 128 registers a thread) spill 920 bytes that way and take their loads as
-// they come: 296 systems, 4 right-hand sides, n = 64 371 -> 276 us, n = 512 8.96 -> 8.21 ms.
+// they come: 296 systems, 4 right-hand sides, n = 64 371 -> 262 us, n = 512 8.87 -> 8.07 ms.
 template <typename T>
 constexpr bool kLoadAhead = sizeof(T) == 8;
 

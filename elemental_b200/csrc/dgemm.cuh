@@ -14,7 +14,8 @@
 // FP64 DMMA (mma.sync m16n8k8 f64): Blackwell's tcgen05 has no f64 kind, and
 // DMMA reaches the FP64 peak (37.2 TFLOP/s measured, DFMA 34.1).
 //
-// Shared-memory layouts (no bank conflicts on any fragment load):
+// Shared-memory layouts (no bank conflicts on any fragment load but K-major
+// A's, whose even rows meet two to a bank, which the DMMA pipe hides):
 //   MN-major operand (m or n contiguous in global): BM/16 boxes of 16 m x
 //     16 k, each [16 k][16 m] (128 B per k row) with the 128B swizzle (16-byte
 //     chunk c of row k at chunk c ^ (k & 7)); one 16-byte load gives two
@@ -49,9 +50,9 @@ constexpr int kStages = 4;
 // warps, so that a CTA alone on its SM (a small product, or the other CTA in
 // its epilogue) still fills the DMMA pipe; MI = 4: four warps with fewer
 // fragment loads per DMMA, the better one for long k loops on a full chip
-// (launch_dgemm chooses).  n = 16384, K = 128 (C full, NT): 2.81 ms with MI = 4,
-// 2.49 with MI = 2 (0.74 of the DMMA rate); n = 8192, K = 2048 (NN): 8.09 and
-// 8.46 ms (0.91, 0.87).  Several tiles per CTA with the next tile's loads under
+// (launch_dgemm chooses).  C full, n = 8192, K = 128 (NT): 0.72 ms with MI = 4, 0.58
+// with MI = 2 (0.80 of the DMMA rate; n = 16384 2.27 ms, 0.82); K = 2048 (NN): 8.00 and
+// 8.13 ms (0.92, 0.91).  Several tiles per CTA with the next tile's loads under
 // the epilogue measured slower (0.67 with four, 0.66 with eight at K = 128): the
 // two CTAs of an SM then stay in step, both in the main loop and both in the
 // epilogue, where one tile per CTA lets them drift apart; two groups of four
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, 2)
     const uint32_t parity = (uint32_t)(kt / kStages) & 1u;
     // warp-uniform outcome: the DMMAs below need the whole warp converged
     // (with MI = 4 the loop is left only at its end: a branch out of it here
-    // costs the NORMAL, NORMAL product 5% at K = 4096, n = 6000 9.03 ms instead of
-    // 8.50; with MI = 2 it gains up to 6% there, n = 1000)
+    // costs the NORMAL, NORMAL product 6% at K = 4096, n = 6000 8.99 ms instead of
+    // 8.45; with MI = 2 it gains up to 6% there, n = 1000)
     ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(&full[s], parity));
     if (MI < 4 && !ok) break;
     const double* sA = reinterpret_cast<const double*>(smem + s * S::kStageBytes);

@@ -4,8 +4,9 @@
 // [c R, c R + R) (R a multiple of 16), the first CT = 32 CW threads of the CTA
 // (its column threads) own local rows t, t + CT, ... (RT of them); the other
 // warps help between the sub-panels.  The panel is processed in 16-column
-// sub-panels; a column thread keeps its rows' sub-panel entries in registers, and each column step rotates them by one as part of its rank-1
-// update, v[k] := v[k + 1] - l u[k], so that register 0 is always the current
+// sub-panels; a column thread keeps its rows' sub-panel entries in registers,
+// and each column step rotates them by one as part of its rank-1 update,
+// v[k] := v[k + 1] - l u[k], so that register 0 is always the current
 // column, the column loop stays rolled, and the columns already done have
 // rotated out as zeros (the winner's u needs no masking).
 //
@@ -18,7 +19,7 @@
 // instruction of it fetched anew in every sub-panel; the rolled form is 85 KB
 // in all.  One 128-column panel, before (unrolled, interchanges in the
 // messages, register FMAs for the trailing columns) and now: m = 128 0.36 ->
-// 0.17 ms, m = 2048 0.354 -> 0.205 ms, m = 8192 0.459 -> 0.325 ms.
+// 0.162 ms, m = 2048 0.354 -> 0.195 ms, m = 8192 0.459 -> 0.308 ms.
 //
 // Pivoting inside a sub-panel is logical: a chosen row is marked done where
 // it is, and every thread tracks the position its rows would have under the
@@ -580,12 +581,12 @@ __global__ void __launch_bounds__(kRpThreads, 1) lu_panel_rp_kernel(int m, int b
 
 // Launch the register-resident panel when m fits one cluster (b <= m <= 16 x
 // 1024 rows with a 16-CTA cluster) and b <= 128.  Returns EGPU_ERR_UNSUPPORTED
-// when it does not apply.  The fewest rows per CTA that fit one cluster: the
-// trailing updates inside the panel get shorter with every CTA (m = 2048:
-// 0.248 ms with 128 rows a CTA, 0.268 with 256, 0.327 with 512, measured on an
-// earlier form of the kernel), the exchange only a little longer.  Four
-// column warps up to 256 rows a CTA and eight above: four warps with four
-// rows a thread measured 0.36 ms at m = 8192 against 0.34 for eight with two.
+// when it does not apply.  The fewest rows per CTA, from 128 on, that fit one
+// cluster: the trailing updates inside the panel get shorter with every CTA,
+// the exchange only a little longer.  128 columns, us, with at most 16, 8 and 4
+// CTAs: m = 1000 191 / 190 / 254, 2048 195 / 251 / 303, 8192 308 / 443 / 847.  Four column
+// warps up to 256 rows a CTA and eight above: four warps with four rows a
+// thread measured 0.36 ms at m = 8192.
 int launch_lu_panel_rp(cudaStream_t st, int m, int b, double* A, long long lda, int* p, int offset, int* image,
                        int* preimage, double* W, int ldw, DevStatus* status, int cluster_max) {
   if (b > 128 || b < 1 || m < b || cluster_max < 1) return EGPU_ERR_UNSUPPORTED;

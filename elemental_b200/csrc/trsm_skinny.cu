@@ -503,7 +503,7 @@ int launch_trsm_skinny(cudaStream_t st, int bwd, int amode, int n, int nrhs, con
   }
   p.epoch = ++seq.epoch;
   const int grid = p.groups * p.gsz;
-  TraceMark tm(st, kTraceSolve, (double)n * n * p.nrhs, 4.0 * (double)n * n + 16.0 * n * p.nrhs);
+  TraceMark tm(st, kTraceSolve, (double)n * n * p.nrhs, 4.0 * (double)n * n * p.groups + 16.0 * n * p.nrhs);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kTsThreads);

@@ -119,7 +119,7 @@ def test_lu_panel_ties_take_the_lowest_row(handle, m):
 
 
 @pytest.mark.parametrize("col", [1, 2, 15, 16, 17, 18, 33, 128, 129, 145])
-def test_cholesky_reports_the_column_in_a_pair(handle, col):
+def test_cholesky_reports_the_failing_column(handle, col):
     n = 145
     A = inputs.spd_ggt(n, 12)
     A[col - 1, col - 1] = -1.0

@@ -283,11 +283,12 @@ static int launch_dgemm_small(cudaStream_t st, bool a_kmajor, bool b_kmajor, int
   // cost more with K, and the engine has one CTA to an SM up to 148 of its tiles:
   // both K-major 576 tiles 0.84 at K = 192 and 1.01 at 256, 1024 1.32 and 1.69, 1444 1.00
   // and 1.36; one K-major, K = 256, 576 0.78, 784 1.12, 1444 1.10.  At most 64 rows or
-  // columns leave half of the engine's tile empty: 64 x 16384, K = 256, 0.68 to 1.00.
+  // 32 columns leave half of the engine's 128 x 64 tile empty: K = 256, 64 x 16384
+  // 0.68 to 1.00 (16384 x 64, which do not, 1.40 with both K-major).
   // In place one wave of CTAs (M = 2048: 22 us in the engine, 10 here; the
   // Cholesky at n = 16384 0.6% slower with the whole range of M here).
   const bool long_k = a_kmajor && b_kmajor ? K > 128 : (a_kmajor || b_kmajor) && K > 192;
-  const int per_sm = long_k && std::min(M, N) > 64 ? 4 : 10;
+  const int per_sm = long_k && M > 64 && N > 32 ? 4 : 10;
   if (!alias_a && !alias_b && t32 / (tri ? 2 : 1) > (long long)per_sm * sms) return EGPU_ERR_UNSUPPORTED;
   if (alias_a && M > 32 * sms) return EGPU_ERR_UNSUPPORTED;
   if (alias_b && N > 32 * sms) return EGPU_ERR_UNSUPPORTED;
